@@ -656,10 +656,9 @@ template <typename S>
 static void launch_periodic(psl_grid* g, int axis) {
   const int nx = g->info.cell_count_x, ny = g->info.cell_count_y, nz = g->info.cell_count_z;
   const int items = (axis == 0 ? ny : nx) * nz;
-  if (axis == 0)
-    periodic_kernel<S, 0><<<blocks_for(items, 256), 256, 0, g->stream>>>(view<S>(g), nx, ny, nz);
-  else
-    periodic_kernel<S, 1><<<blocks_for(items, 256), 256, 0, g->stream>>>(view<S>(g), nx, ny, nz);
+  const dim3 blocks(blocks_for(items, kPeriodicThreads), 2);  // y: the two directions
+  if (axis == 0) periodic_kernel<S, 0><<<blocks, kPeriodicThreads, 0, g->stream>>>(view<S>(g), nx, ny, nz);
+  else periodic_kernel<S, 1><<<blocks, kPeriodicThreads, 0, g->stream>>>(view<S>(g), nx, ny, nz);
 }
 
 static int periodic(psl_grid* g, int axis) {
