@@ -13,10 +13,11 @@
 //     tau_ij = <u_i u_j> - <u>_i <u>_j over the 8 children, S the strain rate of the
 //     filtered velocity (central differences, periodic), in coarse lattice units.
 //
-// Gradients.  The loss is the mean over a batch of (softplus(z) - nu_t*/out_scale)^2.  A
-// block takes 128 samples at a time, one per thread: forward and backward per thread,
-// then the block forms its weight gradients as sums over the 128 samples held in shared
-// memory; blocks write partial gradients that one kernel sums in block order in FP64.
+// Gradients.  The loss is the mean over a batch of (softplus(z) - nu_t*/out_scale)^2.  Each
+// warp takes tiles of 32 samples through the forward pass, the backward pass and the weight
+// gradients as register-tiled matrix products (grad_kernel); blocks write partial gradients
+// that a second kernel sums in a fixed order in FP64, in training together with the Adam
+// update.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -37,9 +38,10 @@ namespace {
 // normalisation (in_shift [10], in_scale [10], out_scale), which training does not change
 constexpr int kW1 = 0, kB1 = 320, kW2 = 352, kB2 = 1376, kW3 = 1408, kB3 = 1440, kTrainable = 1441;
 constexpr int kShift = 1441, kScale = 1451, kOutScale = 1461, kParams = 1462;
-constexpr int kGradThreads = 128;
-constexpr int kGradBlocks = 296;  // 2 x 148 SMs
-constexpr int kRowPad = 33;       // shared rows of 32 values, padded against bank conflicts
+constexpr int kMaxGradWarps = 14;
+constexpr int kGradBlocks = 148;  // one block per SM (159 KB of shared memory at 14 warps)
+constexpr int kTile = 32;         // samples per warp tile
+constexpr int kLd = 36;           // floats per row of 32 samples: consecutive rows 4 banks apart
 
 int fail(int code, const std::string& msg) {
   psl_detail_set_last_error(msg);
@@ -61,159 +63,380 @@ __device__ __forceinline__ uint32_t mix32(uint32_t x) {  // lowbias32 integer ha
   return x;
 }
 
-struct GradShared {
-  float w[kParams];
-  float xn[kGradThreads][kMlpIn];
-  float h1[kGradThreads][kRowPad];
-  float h2[kGradThreads][kRowPad];
-  float d1[kGradThreads][kRowPad];
-  float d2[kGradThreads][kRowPad];
-  float dz[kGradThreads];
-  float loss[kGradThreads];
+// Shared memory of the gradient kernel: the weights once per block, then each warp's
+// activations, transposed (row = unit, column = sample of the tile).
+struct GradWeights {
+  float w1t[kMlpIn][32];  // w1t[i][o] = w1[o][i]
+  float w2t[32][36];      // w2t[k][o] = w2[o][k] (forward; rows padded against bank conflicts in the transposition)
+  float w2[32][32];       // w2[o][k] (backward)
+  float b1[32], b2[32], w3[32];
+  float shift[kMlpIn], scale[kMlpIn];
+  float b3, out_scale;
+  float pad[2];
 };
+struct GradTile {
+  float a[32][kLd];      // relu(z1), later the layer-1 deltas
+  float d[32][kLd];      // layer-2 deltas
+  float x[kMlpIn][kLd];  // normalised features
+};
+static_assert(sizeof(GradWeights) % 16 == 0 && sizeof(GradTile) % 16 == 0, "16-byte aligned rows");
+static_assert(sizeof(GradTile) >= (kTrainable + 1) * sizeof(float), "a warp's gradient fits its tile");
+constexpr size_t grad_smem(int warps) { return sizeof(GradWeights) + (size_t)warps * sizeof(GradTile); }
+
+// Programmatic dependent launch: a kernel's blocks may start before the kernel ahead of it in
+// the stream has finished; grid_wait returns once that one's writes are visible.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+__device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ void st4(float* p, float a, float b, float c, float d) {
+  *reinterpret_cast<float4*>(p) = make_float4(a, b, c, d);
+}
+
+// acc[j][u] += sum over the n rows k of in[k][sample j] * w[k][output u], for the lane's four
+// samples (columns 4 sg ..) and eight outputs (8 og ..), two outputs per packed FMA (each
+// rounded as the scalar one).
+template <int kPitch>
+__device__ __forceinline__ void tile_product(float (&acc)[4][8], const float (*in)[kLd], const float (*w)[kPitch], int n,
+                                             int sg, int og) {
+  float2 p[4][4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+#pragma unroll
+    for (int u = 0; u < 4; ++u) p[j][u] = make_float2(acc[j][2 * u], acc[j][2 * u + 1]);
+#pragma unroll 2
+  for (int k = 0; k < n; ++k) {
+    const float4 sv4 = ld4(&in[k][4 * sg]);
+    const float4 w0 = ld4(&w[k][8 * og]), w1 = ld4(&w[k][8 * og + 4]);
+    const float sv[4] = {sv4.x, sv4.y, sv4.z, sv4.w};
+    const float2 wv[4] = {make_float2(w0.x, w0.y), make_float2(w0.z, w0.w), make_float2(w1.x, w1.y), make_float2(w1.z, w1.w)};
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int u = 0; u < 4; ++u) p[j][u] = __ffma2_rn(wv[u], make_float2(sv[j], sv[j]), p[j][u]);
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      acc[j][2 * u] = p[j][u].x;
+      acc[j][2 * u + 1] = p[j][u].y;
+    }
+}
+// Output u of the lane's tile for its four samples, as row `row` of a transposed buffer.
+__device__ __forceinline__ void store_row(float (*out)[kLd], int row, const float (&acc)[4][8], int u, int sg) {
+  st4(&out[row][4 * sg], acc[0][u], acc[1][u], acc[2][u], acc[3][u]);
+}
+// Sum of v[u] over the eight lanes sg = 0..7 that share og; lane sg gets entry u = sg.
+__device__ __forceinline__ float sum_scatter(const float (&v)[8], int sg) {
+  float a[4], b[2];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const bool up = sg & 4;
+    a[u] = (up ? v[4 + u] : v[u]) + __shfl_xor_sync(0xffffffffu, up ? v[u] : v[4 + u], 4);
+  }
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    const bool up = sg & 2;
+    b[u] = (up ? a[2 + u] : a[u]) + __shfl_xor_sync(0xffffffffu, up ? a[u] : a[2 + u], 2);
+  }
+  const bool up = sg & 1;
+  return (up ? b[1] : b[0]) + __shfl_xor_sync(0xffffffffu, up ? b[0] : b[1], 1);
+}
 
 // Partial gradients of the batch samples [0, count): sample i is row first + i, or a
 // hashed row of [0, n) when `random`.  partial[block][0..kTrainable) gets the block's
-// gradient sums, partial[block][kTrainable] its loss sum.
-__global__ void __launch_bounds__(kGradThreads) grad_kernel(const float* __restrict__ params, const float* __restrict__ X,
-                                                            const float* __restrict__ T, long long n, long long first,
-                                                            long long count, int random, uint32_t seed,
-                                                            float* __restrict__ partial) {
+// gradient sums, partial[block][kTrainable] its loss sum.  Tile t of 32 samples belongs to
+// block t % gridDim.x, warp t / gridDim.x (cyclically).
+//
+// What bounds it: instruction issue and latency, beside the two launches of a step (0.45
+// instructions per cycle and scheduler at 3.5 warps each).  Each lane holds a 4 x 8 tile of
+// the three passes (32 FMAs, two per instruction, from three 16-byte loads) and 8 x 4 of the
+// 32 x 32 weight gradient (128 FMAs from twelve); weight-gradient accumulators stay in
+// registers over all of a warp's tiles.  One training step of 65,536 samples: 60.3 us with one
+// thread per sample (every weight a broadcast load of its own, the weight gradients at two
+// loads per FMA) and three launches; 25.5 us now.  With scalar FMAs 27.7 us; with 64-sample
+// tiles (8 x 8 per lane, 7 warps per SM) 27.4 us without leaving room for the reduction's blocks.
+__global__ void __launch_bounds__(32 * kMaxGradWarps, 1)
+    grad_kernel(const float* params, const float* __restrict__ X, const float* __restrict__ T, long long n, long long first,
+                long long count, int random, uint32_t seed, float* partial) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  GradShared& s = *reinterpret_cast<GradShared*>(smem_raw);
-  for (int i = threadIdx.x; i < kParams; i += blockDim.x) s.w[i] = params[i];
-  __syncthreads();
-  const float inv_count = 1.f / (float)count;
-  const float out_scale = s.w[kOutScale];
-  constexpr int kPer = (kTrainable + kGradThreads - 1) / kGradThreads;
-  float acc[kPer];
-#pragma unroll
-  for (int e = 0; e < kPer; ++e) acc[e] = 0.f;
-  float loss = 0.f;
-  for (long long base = (long long)blockIdx.x * kGradThreads; base < count; base += (long long)gridDim.x * kGradThreads) {
-    const long long i = base + threadIdx.x;
-    const bool valid = i < count;
-    float xn[kMlpIn];
-    float t = 0.f;
+  GradWeights& W = *reinterpret_cast<GradWeights*>(smem_raw);
+  GradTile* tiles = reinterpret_cast<GradTile*>(smem_raw + sizeof(GradWeights));
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  const int sg = lane & 7, og = lane >> 3;
+  GradTile& s = tiles[warp];
+  const int c0 = 4 * sg + og;  // this lane gathers sample c0 of a tile and evaluates its loss
+
+  // the samples do not depend on the kernel ahead (which may still be updating the
+  // parameters): fetch the first tile's before waiting for it
+  float2 raw[kMlpIn / 2] = {};
+  float target = 0.f;
+  bool valid = false;
+  auto gather = [&](long long tile) {
+    const long long i = tile * kTile + c0;
+    valid = i < count;
+    long long row = 0;
     if (valid) {
-      const long long row = random ? (long long)(mix32(seed ^ mix32((uint32_t)i * 2654435761u + (uint32_t)(i >> 32))) % (uint64_t)n)
-                                   : first + i;
-#pragma unroll
-      for (int k = 0; k < kMlpIn; ++k) xn[k] = (X[row * kMlpIn + k] - s.w[kShift + k]) * s.w[kScale + k];
-      t = T[row] / out_scale;
-    } else {
-#pragma unroll
-      for (int k = 0; k < kMlpIn; ++k) xn[k] = 0.f;
-    }
-    // forward
-    float a1[32], a2[32];
-#pragma unroll 4
-    for (int o = 0; o < 32; ++o) {
-      float z = s.w[kB1 + o];
-#pragma unroll
-      for (int k = 0; k < kMlpIn; ++k) z = fmaf(s.w[kW1 + o * kMlpIn + k], xn[k], z);
-      a1[o] = z;
-    }
-#pragma unroll 4
-    for (int o = 0; o < 32; ++o) {
-      float z = s.w[kB2 + o];
-#pragma unroll
-      for (int k = 0; k < 32; ++k) z = fmaf(s.w[kW2 + o * 32 + k], fmaxf(a1[k], 0.f), z);
-      a2[o] = z;
-    }
-    float z = s.w[kB3];
-#pragma unroll
-    for (int k = 0; k < 32; ++k) z = fmaf(s.w[kW3 + k], fmaxf(a2[k], 0.f), z);
-    const float y = z > 20.f ? z : log1pf(expf(z));
-    const float r = valid ? y - t : 0.f;
-    loss += r * r;
-    const float dz = 2.f * r * inv_count / (1.f + expf(-fminf(z, 50.f)));
-    // backward to the hidden layers
-    float d2[32];
-#pragma unroll
-    for (int o = 0; o < 32; ++o) d2[o] = a2[o] > 0.f ? dz * s.w[kW3 + o] : 0.f;
-#pragma unroll 4
-    for (int k = 0; k < 32; ++k) {
-      float g = 0.f;
-#pragma unroll
-      for (int o = 0; o < 32; ++o) g = fmaf(d2[o], s.w[kW2 + o * 32 + k], g);
-      s.d1[threadIdx.x][k] = a1[k] > 0.f ? g : 0.f;
-    }
-#pragma unroll
-    for (int k = 0; k < 32; ++k) {
-      s.h1[threadIdx.x][k] = fmaxf(a1[k], 0.f);
-      s.h2[threadIdx.x][k] = fmaxf(a2[k], 0.f);
-      s.d2[threadIdx.x][k] = d2[k];
-    }
-#pragma unroll
-    for (int k = 0; k < kMlpIn; ++k) s.xn[threadIdx.x][k] = xn[k];
-    s.dz[threadIdx.x] = dz;
-    __syncthreads();
-    // weight gradients: each thread owns entries e = threadIdx.x + kGradThreads * j
-#pragma unroll
-    for (int j = 0; j < kPer; ++j) {
-      const int e = threadIdx.x + kGradThreads * j;
-      if (e >= kTrainable) break;
-      float g = 0.f;
-      if (e < kB1) {
-        const int o = e / kMlpIn, k = e % kMlpIn;
-        for (int b = 0; b < kGradThreads; ++b) g = fmaf(s.d1[b][o], s.xn[b][k], g);
-      } else if (e < kW2) {
-        const int o = e - kB1;
-        for (int b = 0; b < kGradThreads; ++b) g += s.d1[b][o];
-      } else if (e < kB2) {
-        const int o = (e - kW2) / 32, k = (e - kW2) % 32;
-        for (int b = 0; b < kGradThreads; ++b) g = fmaf(s.d2[b][o], s.h1[b][k], g);
-      } else if (e < kW3) {
-        const int o = e - kB2;
-        for (int b = 0; b < kGradThreads; ++b) g += s.d2[b][o];
-      } else if (e < kB3) {
-        const int k = e - kW3;
-        for (int b = 0; b < kGradThreads; ++b) g = fmaf(s.dz[b], s.h2[b][k], g);
-      } else {
-        for (int b = 0; b < kGradThreads; ++b) g += s.dz[b];
+      row = first + i;
+      if (random) {
+        const uint32_t v = mix32(seed ^ mix32((uint32_t)i * 2654435761u + (uint32_t)(i >> 32)));
+        row = n <= 0xffffffffll ? (long long)(v % (uint32_t)n) : (long long)v;
       }
-      acc[j] += g;
     }
-    __syncthreads();
-  }
-  float* out = partial + (size_t)blockIdx.x * (kTrainable + 1);
 #pragma unroll
-  for (int j = 0; j < kPer; ++j) {
-    const int e = threadIdx.x + kGradThreads * j;
-    if (e < kTrainable) out[e] = acc[j];
+    for (int k = 0; k < kMlpIn / 2; ++k) raw[k] = reinterpret_cast<const float2*>(X + row * kMlpIn)[k];
+    target = T[row];
+  };
+  long long tile = blockIdx.x + (long long)gridDim.x * warp;
+  if (tile * kTile < count) gather(tile);
+
+  grid_wait();
+  grid_release();
+  for (int base = threadIdx.x; base < kParams; base += 4 * blockDim.x) {  // one round at 14 warps
+    float v[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const int i = base + c * blockDim.x;
+      v[c] = i < kParams ? __ldcg(params + i) : 0.f;
+    }
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const int i = base + c * blockDim.x;
+      if (i < kB1) W.w1t[i % kMlpIn][i / kMlpIn] = v[c];
+      else if (i < kW2) W.b1[i - kB1] = v[c];
+      else if (i < kB2) {
+        W.w2[(i - kW2) >> 5][(i - kW2) & 31] = v[c];
+        W.w2t[(i - kW2) & 31][(i - kW2) >> 5] = v[c];
+      } else if (i < kW3) W.b2[i - kB2] = v[c];
+      else if (i < kB3) W.w3[i - kW3] = v[c];
+      else if (i < kShift) W.b3 = v[c];
+      else if (i < kScale) W.shift[i - kShift] = v[c];
+      else if (i < kOutScale) W.scale[i - kScale] = v[c];
+      else if (i < kParams) W.out_scale = v[c];
+    }
   }
-  s.loss[threadIdx.x] = loss;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    float l = 0.f;
-    for (int b = 0; b < kGradThreads; ++b) l += s.loss[b];
-    out[kTrainable] = l;
+
+  const float inv_count = 1.f / (float)count;
+  // gradient accumulators over the warp's tiles.  g2: rows o = og + 4 j, columns k = sg + 8 m;
+  // g1: rows k = sg + 8 m, inputs 5 ig + i, half of the samples; b1, b2, w3: entry 8 og + sg
+  const int ig = og & 1, half = og >> 1;
+  float g2[8][4], g1[4][5], gb1 = 0.f, gb2 = 0.f, gw3 = 0.f, gb3 = 0.f, loss = 0.f;
+#pragma unroll
+  for (int m = 0; m < 4; ++m) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) g2[j][m] = 0.f;
+#pragma unroll
+    for (int i = 0; i < 5; ++i) g1[m][i] = 0.f;
+  }
+
+  for (; tile * kTile < count; tile += (long long)gridDim.x * warps) {
+    const bool ok = valid;
+    const float t = target / W.out_scale;
+#pragma unroll
+    for (int k = 0; k < kMlpIn; ++k) {
+      const float v = (k & 1) ? raw[k / 2].y : raw[k / 2].x;
+      s.x[k][c0] = ok ? (v - W.shift[k]) * W.scale[k] : 0.f;
+    }
+    __syncwarp();
+    float acc[4][8], sum[8];
+    // ---- layer 1 ----
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[j][u] = W.b1[8 * og + u];
+    tile_product(acc, s.x, W.w1t, kMlpIn, sg, og);
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[j][u] = fmaxf(acc[j][u], 0.f);
+      store_row(s.a, 8 * og + u, acc, u, sg);
+    }
+    __syncwarp();
+    // ---- layer 2 and the output: z summed over the lane's outputs, then over the four lanes
+    // that share its samples ----
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[j][u] = W.b2[8 * og + u];
+    tile_product(acc, s.a, W.w2t, 32, sg, og);
+    float z[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const float w3 = W.w3[8 * og + u];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) z[j] = fmaf(w3, fmaxf(acc[j][u], 0.f), z[j]);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      z[j] += __shfl_xor_sync(0xffffffffu, z[j], 8);
+      z[j] += __shfl_xor_sync(0xffffffffu, z[j], 16);
+    }
+    // each lane evaluates the loss of the sample it gathered; the four deltas come by shuffles
+    const float zz = (og == 0 ? z[0] : og == 1 ? z[1] : og == 2 ? z[2] : z[3]) + W.b3;
+    const float y = zz > 20.f ? zz : log1pf(expf(zz));
+    const float r = ok ? y - t : 0.f;
+    loss += r * r;
+    const float dz_own = 2.f * r * inv_count / (1.f + expf(-fminf(zz, 50.f)));
+    gb3 += dz_own;
+    float dz[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) dz[j] = __shfl_sync(0xffffffffu, dz_own, sg + 8 * j);
+    // ---- layer-2 deltas, and the sums over samples that need only them ----
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      sum[u] = 0.f;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) sum[u] = fmaf(dz[j], fmaxf(acc[j][u], 0.f), sum[u]);
+    }
+    gw3 += sum_scatter(sum, sg);
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const float w3 = W.w3[8 * og + u];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[j][u] = acc[j][u] > 0.f ? dz[j] * w3 : 0.f;
+      sum[u] = (acc[0][u] + acc[1][u]) + (acc[2][u] + acc[3][u]);
+      store_row(s.d, 8 * og + u, acc, u, sg);
+    }
+    gb2 += sum_scatter(sum, sg);
+    __syncwarp();
+    // ---- weight gradient of layer 2: d (32 x samples) times a^T ----
+#pragma unroll 1
+    for (int c = 0; c < kTile; c += 4) {
+      float4 av[4];
+#pragma unroll
+      for (int m = 0; m < 4; ++m) av[m] = ld4(&s.a[sg + 8 * m][c]);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float4 dv = ld4(&s.d[og + 4 * j][c]);
+#pragma unroll
+        for (int m = 0; m < 4; ++m)
+          g2[j][m] = fmaf(dv.w, av[m].w, fmaf(dv.z, av[m].z, fmaf(dv.y, av[m].y, fmaf(dv.x, av[m].x, g2[j][m]))));
+      }
+    }
+    // ---- layer-1 deltas ----
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[j][u] = 0.f;
+    tile_product(acc, s.d, W.w2, 32, sg, og);
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const float4 a4 = ld4(&s.a[8 * og + u][4 * sg]);
+      const float av[4] = {a4.x, a4.y, a4.z, a4.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[j][u] = av[j] > 0.f ? acc[j][u] : 0.f;
+      sum[u] = (acc[0][u] + acc[1][u]) + (acc[2][u] + acc[3][u]);
+    }
+    gb1 += sum_scatter(sum, sg);
+    __syncwarp();  // every lane has read the activations that the deltas replace
+#pragma unroll
+    for (int u = 0; u < 8; ++u) store_row(s.a, 8 * og + u, acc, u, sg);
+    __syncwarp();
+    // the next tile's samples arrive during the last product
+    const long long next = tile + (long long)gridDim.x * warps;
+    if (next * kTile < count) gather(next);
+    // ---- weight gradient of layer 1: d1 (32 x samples) times x^T ----
+#pragma unroll 1
+    for (int c = kTile / 2 * half; c < kTile / 2 * (half + 1); c += 4) {
+      float4 dv[4];
+#pragma unroll
+      for (int m = 0; m < 4; ++m) dv[m] = ld4(&s.a[sg + 8 * m][c]);
+#pragma unroll
+      for (int i = 0; i < 5; ++i) {
+        const float4 xv = ld4(&s.x[5 * ig + i][c]);
+#pragma unroll
+        for (int m = 0; m < 4; ++m)
+          g1[m][i] = fmaf(dv[m].w, xv.w, fmaf(dv[m].z, xv.z, fmaf(dv[m].y, xv.y, fmaf(dv[m].x, xv.x, g1[m][i]))));
+      }
+    }
+    __syncwarp();  // the tile's buffers are free for the next one
+  }
+
+  // ---- the warp's sums, laid out like the parameters, into its own tile buffer ----
+  float* mine = reinterpret_cast<float*>(&s);
+#pragma unroll
+  for (int j = 0; j < 8; ++j)
+#pragma unroll
+    for (int m = 0; m < 4; ++m) mine[kW2 + (og + 4 * j) * 32 + sg + 8 * m] = g2[j][m];
+#pragma unroll
+  for (int m = 0; m < 4; ++m)
+#pragma unroll
+    for (int i = 0; i < 5; ++i) {
+      const float v = g1[m][i] + __shfl_xor_sync(0xffffffffu, g1[m][i], 16);
+      if (half == 0) mine[kW1 + (sg + 8 * m) * kMlpIn + 5 * ig + i] = v;
+    }
+  mine[kB1 + 8 * og + sg] = gb1;
+  mine[kB2 + 8 * og + sg] = gb2;
+  mine[kW3 + 8 * og + sg] = gw3;
+#pragma unroll
+  for (int d = 1; d < 32; d *= 2) {
+    gb3 += __shfl_xor_sync(0xffffffffu, gb3, d);
+    loss += __shfl_xor_sync(0xffffffffu, loss, d);
+  }
+  if (lane == 0) {
+    mine[kB3] = gb3;
+    mine[kTrainable] = loss;
+  }
+  __syncthreads();
+  float* out = partial + (size_t)blockIdx.x * (kTrainable + 1);
+  for (int e = threadIdx.x; e <= kTrainable; e += blockDim.x) {
+    float v = 0.f;
+    for (int w = 0; w < warps; ++w) v += reinterpret_cast<const float*>(&tiles[w])[e];
+    out[e] = v;
   }
 }
 
-// grad[e] = sum over blocks (in block order, FP64) of partial[block][e]; grad[kTrainable] is
-// the mean loss.
-__global__ void reduce_kernel(const float* __restrict__ partial, int blocks, long long count, double* __restrict__ grad) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e > kTrainable) return;
+// grad[e] = sum over blocks of partial[block][e] in FP64, grad[kTrainable] the mean loss; with
+// kAdam also the Adam update of the parameter.  Eight entries (one 32-byte sector of a block's
+// row) per block and 16 groups of threads that take every 16th row each, then the 16 sums in
+// order.  One thread per entry summing all rows kept six blocks busy with a serial chain of
+// loads (16.3 us at 296 rows, Adam a launch of its own at 4.2 us).  128 threads of at most 32
+// registers fit beside a block of grad_kernel, so each of the two kernels is resident when
+// the one ahead of it ends.
+struct AdamParams {
+  float* params;
+  float* m;
+  float* v;
+  float lr, beta1, beta2, eps;
+  int step;
+};
+constexpr int kReduceEntries = 8, kReduceGroups = 16;
+template <bool kAdam>
+__global__ void __launch_bounds__(kReduceEntries * kReduceGroups, 16)
+    reduce_kernel(const float* partial, int blocks, long long count, double* grad, AdamParams ad) {
+  __shared__ double part[kReduceGroups][kReduceEntries];
+  const int entry = threadIdx.x % kReduceEntries, group = threadIdx.x / kReduceEntries;
+  const int e = blockIdx.x * kReduceEntries + entry;
+  grid_wait();
+  grid_release();
+  constexpr int kRows = (kGradBlocks + kReduceGroups - 1) / kReduceGroups;
+  float v[kRows];
+#pragma unroll
+  for (int r = 0; r < kRows; ++r) {
+    const int b = group + r * kReduceGroups;
+    v[r] = e <= kTrainable && b < blocks ? __ldcg(partial + (size_t)b * (kTrainable + 1) + e) : 0.f;
+  }
   double s = 0.0;
-  for (int b = 0; b < blocks; ++b) s += (double)partial[(size_t)b * (kTrainable + 1) + e];
+#pragma unroll
+  for (int r = 0; r < kRows; ++r) s += (double)v[r];
+  part[group][entry] = s;
+  __syncthreads();
+  if (group != 0 || e > kTrainable) return;
+  s = 0.0;
+#pragma unroll
+  for (int w = 0; w < kReduceGroups; ++w) s += part[w][entry];
   grad[e] = e == kTrainable ? s / (double)count : s;
-}
-
-__global__ void adam_kernel(float* __restrict__ params, float* __restrict__ m, float* __restrict__ v,
-                            const double* __restrict__ grad, float lr, float beta1, float beta2, float eps, int step) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= kTrainable) return;
-  const float g = (float)grad[e];
-  const float mm = beta1 * m[e] + (1.f - beta1) * g;
-  const float vv = beta2 * v[e] + (1.f - beta2) * g * g;
-  m[e] = mm;
-  v[e] = vv;
-  const float mh = mm / (1.f - powf(beta1, (float)step));
-  const float vh = vv / (1.f - powf(beta2, (float)step));
-  params[e] -= lr * mh / (sqrtf(vh) + eps);
+  if (!kAdam || e >= kTrainable) return;
+  const float g = (float)s;
+  const float mm = ad.beta1 * ad.m[e] + (1.f - ad.beta1) * g;
+  const float vv = ad.beta2 * ad.v[e] + (1.f - ad.beta2) * g * g;
+  ad.m[e] = mm;
+  ad.v[e] = vv;
+  const float mh = mm / (1.f - powf(ad.beta1, (float)ad.step));
+  const float vh = vv / (1.f - powf(ad.beta2, (float)ad.step));
+  ad.params[e] -= ad.lr * mh / (sqrtf(vh) + ad.eps);
 }
 
 // ---- samples from a fine periodic box ----
@@ -353,14 +576,39 @@ struct psl_sgs_trainer {
 
 namespace {
 
-int run_gradient(psl_sgs_trainer* t, long long first, long long count, int random, uint32_t seed) {
-  const size_t smem = sizeof(GradShared);
-  TRAIN_CUDA(cudaFuncSetAttribute(grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const int blocks = (int)std::min<long long>(kGradBlocks, (count + kGradThreads - 1) / kGradThreads);
-  grad_kernel<<<blocks, kGradThreads, smem, t->stream>>>(t->params, t->X, t->T, t->count, first, count, random, seed,
-                                                         t->partial);
-  reduce_kernel<<<(kTrainable + 1 + 255) / 256, 256, 0, t->stream>>>(t->partial, blocks, count, t->grad);
-  TRAIN_CUDA(cudaGetLastError());
+// A launch that may start while the kernel ahead of it in the stream is finishing (both
+// kernels wait for that one, grid_wait, before they touch anything it writes).
+template <typename... P, typename... A>
+cudaError_t launch_dependent(void (*kernel)(P...), unsigned int blocks, unsigned int threads, size_t smem, cudaStream_t stream,
+                             A... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(blocks);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+// One warp per 32-sample tile while that many warps fit (14 per SM), so that a batch of 65,536
+// samples is one tile per warp on 148 x 14 warps and a small batch spreads over the SMs.
+int run_gradient(psl_sgs_trainer* t, long long first, long long count, int random, uint32_t seed, const AdamParams* adam) {
+  const long long tiles = (count + kTile - 1) / kTile;
+  const int blocks = (int)std::min<long long>(kGradBlocks, tiles);
+  const int warps = (int)std::min<long long>(kMaxGradWarps, (tiles + blocks - 1) / blocks);
+  TRAIN_CUDA(launch_dependent(grad_kernel, blocks, 32 * warps, grad_smem(warps), t->stream, (const float*)t->params,
+                              (const float*)t->X, (const float*)t->T, t->count, first, count, random, seed, t->partial));
+  const unsigned int nb = (kTrainable + kReduceEntries) / kReduceEntries, threads = kReduceEntries * kReduceGroups;
+  if (adam)
+    TRAIN_CUDA(launch_dependent(reduce_kernel<true>, nb, threads, 0, t->stream, (const float*)t->partial, blocks,
+                                count, t->grad, *adam));
+  else
+    TRAIN_CUDA(launch_dependent(reduce_kernel<false>, nb, threads, 0, t->stream, (const float*)t->partial, blocks,
+                                count, t->grad, AdamParams{}));
   return PSL_OK;
 }
 
@@ -386,6 +634,8 @@ int psl_sgs_trainer_create(long long capacity, psl_sgs_trainer** out) {
   if (e == cudaSuccess) e = cudaMemset(t->params, 0, kParams * sizeof(float));
   if (e == cudaSuccess) e = cudaMemset(t->m, 0, kTrainable * sizeof(float));
   if (e == cudaSuccess) e = cudaMemset(t->v, 0, kTrainable * sizeof(float));
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)grad_smem(kMaxGradWarps));
   if (e != cudaSuccess) {
     const std::string msg = std::string("psl_sgs_trainer_create: ") + cudaGetErrorString(e);
     cudaGetLastError();
@@ -509,7 +759,7 @@ int psl_sgs_trainer_gradient(psl_sgs_trainer* t, long long first, long long coun
   if (!t || first < 0 || count <= 0 || first + count > t->count)
     return fail(PSL_ERR_INVALID, "psl_sgs_trainer_gradient: bad range");
   DeviceGuard dg(t->device);
-  int rc = run_gradient(t, first, count, 0, 0);
+  int rc = run_gradient(t, first, count, 0, 0, nullptr);
   if (rc) return rc;
   std::vector<double> g(kTrainable + 1);
   TRAIN_CUDA(cudaMemcpyAsync(g.data(), t->grad, (kTrainable + 1) * sizeof(double), cudaMemcpyDeviceToHost, t->stream));
@@ -528,10 +778,9 @@ int psl_sgs_trainer_train(psl_sgs_trainer* t, int steps, int batch, float lr, un
   DeviceGuard dg(t->device);
   for (int s = 0; s < steps; ++s) {
     ++t->step;
-    int rc = run_gradient(t, 0, batch, 1, seed * 0x9e3779b9u + (uint32_t)t->step);
+    const AdamParams adam{t->params, t->m, t->v, lr, 0.9f, 0.999f, 1e-8f, t->step};
+    int rc = run_gradient(t, 0, batch, 1, seed * 0x9e3779b9u + (uint32_t)t->step, &adam);
     if (rc) return rc;
-    adam_kernel<<<(kTrainable + 255) / 256, 256, 0, t->stream>>>(t->params, t->m, t->v, t->grad, lr, 0.9f, 0.999f,
-                                                                  1e-8f, t->step);
   }
   TRAIN_CUDA(cudaGetLastError());
   if (last_loss) {
