@@ -15,6 +15,7 @@
 #include "psl.h"
 #include "psl_internal.h"
 #include "psl_kernels.cuh"
+#include "psl_launch.cuh"
 #include "psl_rowmap.h"
 
 using namespace psl;
@@ -43,7 +44,7 @@ __attribute__((visibility("hidden"))) void psl_detail_set_last_error(const std::
     if (!(cond)) return fail(code, msg); \
   } while (0)
 
-static constexpr int kForceBlocks = 512;
+static constexpr int kForceBlocks = 512;  // below 2^16 (force_kernel's block count)
 
 template <typename S>
 static GridView<S> view(const psl_grid* g) {
@@ -174,7 +175,8 @@ int psl_grid_create_ex(const psl_info* info, int storage, unsigned int flags, ps
   }
   if (e == cudaSuccess) e = cudaMalloc(&g->marker, g->stride);
   if (e == cudaSuccess) e = cudaMalloc(&g->health, 4 * sizeof(unsigned int));
-  if (e == cudaSuccess) e = cudaMalloc(&g->scratch, (kForceBlocks * 3 + 3) * sizeof(double));
+  if (e == cudaSuccess) e = cudaMalloc(&g->scratch, (kForceBlocks * 3 + 4) * sizeof(double));
+  if (e == cudaSuccess) e = cudaMemset(g->scratch, 0, (kForceBlocks * 3 + 4) * sizeof(double));
   if (e == cudaSuccess) e = cudaMemset(g->marker, make_marker(kFluid, 0), g->stride);
   if (e == cudaSuccess) e = cudaMemset(g->health, 0, 4 * sizeof(unsigned int));
   if (e == cudaSuccess) e = cudaMemset2D(g->f, g->f_stride * elem, 0, (g->f_twice ? (size_t)n : g->stride) * elem, 27);
@@ -545,7 +547,9 @@ static cudaError_t launch_step(psl_grid* g, bool held_nu, const ThreadRange& ran
   p.range = range;
   const unsigned int blocks = blocks_for(range.count, kStepThreads);
   const int addr = 27 * g->f_stride + g->n >= (1ull << 32) ? kAddrView : g->f_twice ? kAddrFlat : kAddrIndex;
-  auto launch = [&](auto kernel) { kernel<<<blocks, kStepThreads, 0, g->stream>>>(p); };
+  const bool dependent = !kCollidesOnG<S> && !stream_capturing(g->stream);
+  cudaError_t e = cudaSuccess;
+  auto launch = [&](auto kernel) { e = launch_dependent(dependent, kernel, dim3(blocks), kStepThreads, 0, g->stream, p); };
   if constexpr (kCollidesOnG<S>) {
     const int rate = held_nu ? kRateNuField : g->cs_field ? kRateCsField : kRateUniform;
     auto pick = [&](auto addr_tag) {
@@ -562,7 +566,7 @@ static cudaError_t launch_step(psl_grid* g, bool held_nu, const ThreadRange& ran
     else if (addr == kAddrFlat) launch(step_kernel<S, kAddrFlat>);
     else launch(step_kernel<S, kAddrIndex>);
   }
-  return cudaGetLastError();
+  return e;
 }
 
 // The update of the threads in `range` for the plain and the learned-closure paths (the
@@ -592,7 +596,7 @@ int psl_apply_local_cell_update(psl_grid* g) {
               "learned closure");
     PSL_CHECK(g->storage != kStoreF64 && 27ull * g->f_stride + g->n < (1ull << 32) && 27ull * g->stride + g->n < (1ull << 32), PSL_ERR_INVALID,
               "psl_apply_local_cell_update: scalar transport needs FP32/FP16/BF16 storage");
-    with_storage(g->storage, [&](auto s) {
+    PSL_CUDA(with_storage(g->storage, [&](auto s) {
       using S = decltype(s);
       if constexpr (S::kind != kStoreF64) {
         ScalarParams<S> sp;
@@ -612,11 +616,11 @@ int psl_apply_local_cell_update(psl_grid* g) {
         }
         sp.givenT = g->givenT;
         sp.tauT = g->tauT;
-        step_scalar_kernel<S><<<blocks_for(g->n, kStepThreads), kStepThreads, 0, g->stream>>>(sp);
+        return launch_dependent(false, step_scalar_kernel<S>, dim3(blocks_for(g->n, kStepThreads)),
+                                kStepThreads, 0, g->stream, sp);
       }
-      return 0;
-    });
-    PSL_CUDA(cudaGetLastError());
+      return cudaErrorInvalidValue;
+    }));
     return PSL_OK;
   }
   if (g->mlp) {
@@ -629,7 +633,7 @@ int psl_apply_local_cell_update(psl_grid* g) {
   if (custom) {
     PSL_CHECK(g->storage != kStoreF64 && 27ull * g->f_stride + g->n < (1ull << 32), PSL_ERR_INVALID,
               "psl_apply_local_cell_update: forcing and moving walls need FP32/FP16/BF16 storage");
-    with_storage(g->storage, [&](auto s) {
+    PSL_CUDA(with_storage(g->storage, [&](auto s) {
       using S = decltype(s);
       if constexpr (S::kind != kStoreF64) {
         CustomParams<S> cp;
@@ -642,33 +646,29 @@ int psl_apply_local_cell_update(psl_grid* g) {
         cp.base.rx = relaxation<float>(g);
         cp.base.health = g->health;
         cp.body = g->body;
-        step_custom_kernel<S><<<blocks_for(g->n, kStepThreads), kStepThreads, 0, g->stream>>>(cp);
+        return launch_dependent(false, step_custom_kernel<S>, dim3(blocks_for(g->n, kStepThreads)),
+                                kStepThreads, 0, g->stream, cp);
       }
-      return 0;
-    });
-    PSL_CUDA(cudaGetLastError());
+      return cudaErrorInvalidValue;
+    }));
     return PSL_OK;
   }
   return update_cells(g, full_range(g->n));
 }
 
 template <typename S>
-static void launch_periodic(psl_grid* g, int axis) {
+static cudaError_t launch_periodic(psl_grid* g, int axis) {
   const int nx = g->info.cell_count_x, ny = g->info.cell_count_y, nz = g->info.cell_count_z;
   const int items = (axis == 0 ? ny : nx) * nz;
   const dim3 blocks(blocks_for(items, kPeriodicThreads), 2);  // y: the two directions
-  if (axis == 0) periodic_kernel<S, 0><<<blocks, kPeriodicThreads, 0, g->stream>>>(view<S>(g), nx, ny, nz);
-  else periodic_kernel<S, 1><<<blocks, kPeriodicThreads, 0, g->stream>>>(view<S>(g), nx, ny, nz);
+  return launch_dependent(!stream_capturing(g->stream), axis == 0 ? periodic_kernel<S, 0> : periodic_kernel<S, 1>, blocks,
+                          kPeriodicThreads, 0, g->stream, view<S>(g), nx, ny, nz);
 }
 
 static int periodic(psl_grid* g, int axis) {
   PSL_CHECK(g, PSL_ERR_INVALID, "psl_apply_bc_periodic: null grid");
   DeviceGuard dg(g->device);
-  with_storage(g->storage, [&](auto s) {
-    launch_periodic<decltype(s)>(g, axis);
-    return 0;
-  });
-  PSL_CUDA(cudaGetLastError());
+  PSL_CUDA(with_storage(g->storage, [&](auto s) { return launch_periodic<decltype(s)>(g, axis); }));
   return PSL_OK;
 }
 int psl_apply_bc_periodic_x(psl_grid* g) { return periodic(g, 0); }
@@ -882,16 +882,10 @@ int psl_update_grid(psl_grid** grids, int levels, int level) {
 }
 
 // ---- reductions ----
-template <typename S>
-static void launch_force(psl_grid* g, int i0, int j0, int k0, int si, int sj, int sk, int nb) {
-  force_partial_kernel<S><<<nb, 256, 0, g->stream>>>(view<S>(g), g->marker, g->info.cell_count_x,
-                                                     g->info.cell_count_y, i0, j0, k0, si, sj, sk, g->scratch);
-}
-
-// Enqueues the momentum-exchange force of the sphere's box on the grid's stream; the
-// result (3 doubles) lands in `force3` (device or pinned host memory) when the stream
-// reaches the copy.  Returns 1 with nothing enqueued when the box is empty.
-static int enqueue_sphere_force(psl_grid* g, const psl_sphere_case* sc, double* force3, cudaMemcpyKind kind) {
+// Enqueues the momentum-exchange force of the sphere's box on the grid's stream, written to
+// `out` (3 doubles the device can write).  Returns 1 with nothing enqueued when the box is
+// empty.
+static int enqueue_sphere_force(psl_grid* g, const psl_sphere_case* sc, double* out) {
   const psl_info& I = g->info;
   // bounding box as getSphereDrag computes it (flowAroundSphereMainSingle.cu:105-110)
   int i0 = (int)((sc->sphere_x - sc->sphere_r - I.ox) / I.res);
@@ -904,14 +898,15 @@ static int enqueue_sphere_force(psl_grid* g, const psl_sphere_case* sc, double* 
   i1 = std::min(i1, I.cell_count_x); j1 = std::min(j1, I.cell_count_y); k1 = std::min(k1, I.cell_count_z);
   if (i1 <= i0 || j1 <= j0 || k1 <= k0) return 1;
   const int si = i1 - i0, sj = j1 - j0, sk = k1 - k0;
-  const int nb = (int)std::min<long long>(kForceBlocks, ((long long)si * sj * sk + 255) / 256);
-  with_storage(g->storage, [&](auto s) {
-    launch_force<decltype(s)>(g, i0, j0, k0, si, sj, sk, nb);
-    return 0;
-  });
-  force_final_kernel<<<1, 256, 0, g->stream>>>(g->scratch, nb, g->scratch + kForceBlocks * 3);
-  PSL_CUDA(cudaGetLastError());
-  PSL_CUDA(cudaMemcpyAsync(force3, g->scratch + kForceBlocks * 3, 3 * sizeof(double), kind, g->stream));
+  const int nb = (int)std::min<long long>(kForceBlocks, ((long long)si * sj * sk + kForceThreads - 1) / kForceThreads);
+  g->force_calls = g->force_calls % 0xffffu + 1;  // 1 .. 65535
+  unsigned int* done = reinterpret_cast<unsigned int*>(g->scratch + kForceBlocks * 3 + 3);
+  PSL_CUDA(with_storage(g->storage, [&](auto s) {
+    using S = decltype(s);
+    return launch_dependent(!stream_capturing(g->stream), force_kernel<S>, dim3(nb), kForceThreads, 0, g->stream, view<S>(g),
+                            g->marker, I.cell_count_x, I.cell_count_y, i0, j0, k0, si, sj, sk, g->scratch, done,
+                            g->force_calls, out);
+  }));
   return PSL_OK;
 }
 
@@ -919,23 +914,42 @@ int psl_sphere_force(psl_grid* g, const psl_sphere_case* sc, double* force3) {
   PSL_CHECK(g && sc && force3, PSL_ERR_INVALID, "psl_sphere_force: null argument");
   DeviceGuard dg(g->device);
   force3[0] = force3[1] = force3[2] = 0.0;
-  const int rc = enqueue_sphere_force(g, sc, force3, cudaMemcpyDeviceToHost);
+  double* result = g->scratch + kForceBlocks * 3;
+  const int rc = enqueue_sphere_force(g, sc, result);
   if (rc == 1) return PSL_OK;
   if (rc != PSL_OK) return rc;
+  PSL_CUDA(cudaMemcpyAsync(force3, result, 3 * sizeof(double), cudaMemcpyDeviceToHost, g->stream));
   PSL_CUDA(cudaStreamSynchronize(g->stream));
   return PSL_OK;
+}
+
+// The address at which a kernel on `device` can write the three doubles at p: p in that
+// device's memory, managed memory or pinned host memory mapped into it; null when p has to be
+// reached by a copy (another device's memory, pageable memory, a misaligned address).
+static double* device_writable(double* p, int device) {
+  if (reinterpret_cast<uintptr_t>(p) % alignof(double) != 0) return nullptr;
+  cudaPointerAttributes a{};
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  if (a.type == cudaMemoryTypeUnregistered || (a.type == cudaMemoryTypeDevice && a.device != device)) return nullptr;
+  return static_cast<double*>(a.devicePointer);
 }
 
 int psl_sphere_force_async(psl_grid* g, const psl_sphere_case* sc, double* force3) {
   PSL_CHECK(g && sc && force3, PSL_ERR_INVALID, "psl_sphere_force_async: null argument");
   DeviceGuard dg(g->device);
-  const int rc = enqueue_sphere_force(g, sc, force3, cudaMemcpyDefault);
+  double* result = g->scratch + kForceBlocks * 3;
+  double* out = device_writable(force3, g->device);
+  const int rc = enqueue_sphere_force(g, sc, out ? out : result);
   if (rc == 1) {  // empty box: zeros, in stream order like the non-empty case
-    PSL_CUDA(cudaMemsetAsync(g->scratch + kForceBlocks * 3, 0, 3 * sizeof(double), g->stream));
-    PSL_CUDA(cudaMemcpyAsync(force3, g->scratch + kForceBlocks * 3, 3 * sizeof(double), cudaMemcpyDefault, g->stream));
-    return PSL_OK;
+    PSL_CUDA(cudaMemsetAsync(result, 0, 3 * sizeof(double), g->stream));
+  } else if (rc != PSL_OK || out) {
+    return rc;
   }
-  return rc;
+  PSL_CUDA(cudaMemcpyAsync(force3, result, 3 * sizeof(double), cudaMemcpyDefault, g->stream));
+  return PSL_OK;
 }
 
 // ---- data movement ----

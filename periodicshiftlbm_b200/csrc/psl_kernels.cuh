@@ -14,6 +14,7 @@
 #include "psl_collision_g.cuh"
 #include "psl_hooks.cuh"
 #include "psl_lattice.cuh"
+#include "psl_launch.cuh"
 #include "psl_storage.cuh"
 
 namespace psl {
@@ -357,11 +358,17 @@ __device__ __forceinline__ void update_one_cell_g(const StepParams<S>& p, uint32
   if (collides) store_for<StoredOf<S>, kAddr>(p, cell, g);
 }
 
-// One thread per cell: FP32 / FP64 storage.
+// One thread per cell: FP32 / FP64 storage.  A dependent launch (psl_launch.cuh): small grids
+// are a chain of short launches, and the next one's blocks start up while this one's last ones
+// finish (64x32x32 grid: 8.2 -> 7.2 us per step).  The 16-bit kernels are launched the ordinary
+// way: at their 64 registers the ordinary loads a dependent launch needs, in place of the
+// read-only path, spilled 116 bytes (256x128x128 refined sphere, FP16: 233.6 -> 240.0 us).
 template <typename S, int kAddr>
 __global__ void __launch_bounds__(kStepThreads) step_kernel(const __grid_constant__ StepParams<S> p) {
   static_assert(!kCollidesOnG<S>, "16-bit storage runs step_kernel_g");
-  const uint32_t u = blockIdx.x * kStepThreads + threadIdx.x;
+  uint32_t u = blockIdx.x * kStepThreads + threadIdx.x;
+  grid_wait(u);
+  grid_release();
   if (u >= p.range.count) return;
   const uint32_t cell = cell_of_thread(range_thread(p.range, u), p.rot, p.g.n);
   update_one_cell<S, kAddr>(p, cell, p.marker[cell]);
@@ -668,8 +675,10 @@ __global__ void __launch_bounds__(kPeriodicThreads) periodic_kernel(const __grid
                                                                     int nz) {
   const int t = blockIdx.x * kPeriodicThreads + threadIdx.x;
   const int na = Axis == 0 ? ny : nx;
-  if (t >= na * nz) return;
   const int a = t % na, k = t / na;
+  grid_wait();
+  grid_release();
+  if (t >= na * nz) return;
   uint32_t left, right;
   if (Axis == 0) {
     left = ((uint32_t)k * ny + a) * nx;
@@ -913,12 +922,15 @@ __global__ void __launch_bounds__(kCoarseFineThreads) coarse_fine_kernel(const _
 // ------------------------------------------------------------------------------------------
 // momentum-exchange force on the solid cells of a box, FP64
 // (getSphereDrag, flowAroundSphereMainSingle.cu:99-156; per cell rho*(u - u_bounced))
-// Deterministic: per-block partial sums, then one block sums them in block order.
+// Deterministic: per-block partial sums, added in block order.
 // ------------------------------------------------------------------------------------------
+constexpr int kForceThreads = 256;
+
+// The block's share of the box [i0, i0 + si) x ..., reduced over its threads into partial
+// (entries 3 blockIdx.x ..); thread 0 writes them.
 template <typename S>
-__global__ void __launch_bounds__(256) force_partial_kernel(GridView<S> g, const uint8_t* marker, int nx, int ny,
-                                                            int i0, int j0, int k0, int si, int sj, int sk,
-                                                            double* partial) {
+__device__ __forceinline__ void force_partial(const GridView<S>& g, const uint8_t* marker, int nx, int ny, int i0, int j0,
+                                              int k0, int si, int sj, int sk, double* partial) {
   const uint32_t total = (uint32_t)si * sj * sk;
   double acc[3] = {0.0, 0.0, 0.0};
   for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
@@ -942,7 +954,7 @@ __global__ void __launch_bounds__(256) force_partial_kernel(GridView<S> g, const
     acc[1] += rho * (jy / rho - by / rho);
     acc[2] += rho * (jz / rho - bz / rho);
   }
-  __shared__ double red[3][256];
+  __shared__ double red[3][kForceThreads];
   for (int c = 0; c < 3; ++c) red[c][threadIdx.x] = acc[c];
   __syncthreads();
   for (int s = blockDim.x / 2; s > 0; s >>= 1) {
@@ -952,6 +964,62 @@ __global__ void __launch_bounds__(256) force_partial_kernel(GridView<S> g, const
   }
   if (threadIdx.x == 0)
     for (int c = 0; c < 3; ++c) partial[blockIdx.x * 3 + c] = red[c][0];
+}
+
+template <typename S>
+__global__ void __launch_bounds__(kForceThreads) force_partial_kernel(GridView<S> g, const uint8_t* marker, int nx, int ny,
+                                                                      int i0, int j0, int k0, int si, int sj, int sk,
+                                                                      double* partial) {
+  force_partial(g, marker, nx, ny, i0, j0, k0, si, sj, sk, partial);
+}
+
+// The force in one launch: the block that finishes last adds the partial sums in block order
+// (the sums and bits of force_partial_kernel followed by force_final_kernel) and writes the
+// three components to `out`, device memory or mapped host memory, so no copy follows.  A step
+// of the 128x64x64 sphere with its drag read every step took 42.9 us with two kernels and a
+// 24-byte copy behind the update; 33.1 us with this
+// kernel, both as dependent launches (37.2 us without).
+// `done`: blocks finished in the low 16 bits, the call's number above them: a count left by
+// another call starts anew, and the last block clears it (a replayed capture repeats its number).
+template <typename S>
+__global__ void __launch_bounds__(kForceThreads)
+    force_kernel(const __grid_constant__ GridView<S> g, const uint8_t* marker, int nx, int ny, int i0, int j0, int k0, int si,
+                 int sj, int sk, double* partial, unsigned int* done, unsigned int call, double* out) {
+  constexpr int kChunk = 256;  // blocks per staged chunk
+  __shared__ double stage[kChunk * 3];
+  __shared__ bool last;
+  grid_wait();
+  grid_release();
+  force_partial(g, marker, nx, ny, i0, j0, k0, si, sj, sk, partial);
+  if (threadIdx.x == 0) {
+    __threadfence();  // the partial sums before the count
+    unsigned int seen = *(volatile unsigned int*)done, next;
+    for (;;) {
+      next = (seen >> 16) == call ? seen + 1 : (call << 16) + 1;
+      const unsigned int old = atomicCAS(done, seen, next);
+      if (old == seen) break;
+      seen = old;
+    }
+    last = (next & 0xffffu) == gridDim.x;
+    if (last) {
+      *done = 0;
+      __threadfence();
+    }
+  }
+  __syncthreads();
+  if (!last) return;
+  const int nblocks = gridDim.x;
+  double s = 0.0;
+  for (int b0 = 0; b0 < nblocks; b0 += kChunk) {
+    const int nb = min(kChunk, nblocks - b0);
+    for (int i = threadIdx.x; i < nb * 3; i += kForceThreads) stage[i] = __ldcg(partial + b0 * 3 + i);
+    __syncthreads();
+    if (threadIdx.x < 3)
+#pragma unroll 8
+      for (int b = 0; b < nb; ++b) s += stage[b * 3 + threadIdx.x];
+    __syncthreads();
+  }
+  if (threadIdx.x < 3) out[threadIdx.x] = s;
 }
 
 // The partial sums added in block order by one thread (deterministic); every thread of the

@@ -23,7 +23,6 @@ using namespace psl;
 namespace {
 
 constexpr int kNoAllocBlocks = 1024;          // partial sums the fixed scratch holds
-constexpr int kNoAllocThreads = 256;          // threads per block of the partial-sum kernel
 constexpr long long kNoAllocCellsPerBlock = 4096;
 // Largest box accepted: kNoAllocBlocks blocks of kNoAllocCellsPerBlock cells (4,194,304).
 constexpr long long kNoAllocMaxBoxCells = kNoAllocBlocks * kNoAllocCellsPerBlock;
@@ -117,7 +116,7 @@ int psl_momentum_exchange_force_noalloc(const float* populations, long long row_
   // Every block writes its own partial before the final kernel reads it, so the scratch
   // needs no clearing between calls.
   const int nb = cells == 0 ? 1 : (int)((cells + kNoAllocCellsPerBlock - 1) / kNoAllocCellsPerBlock);
-  force_partial_kernel<StoreF32><<<nb, kNoAllocThreads, 0, stream>>>(
+  force_partial_kernel<StoreF32><<<nb, kForceThreads, 0, stream>>>(
       g, markers, nx, ny, box_lo3[0], box_lo3[1], box_lo3[2], box_hi3[0] - box_lo3[0], box_hi3[1] - box_lo3[1],
       box_hi3[2] - box_lo3[2], scratch);
   force_final_kernel<<<1, 256, 0, stream>>>(scratch, nb, force3);

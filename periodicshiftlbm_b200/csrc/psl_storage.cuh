@@ -18,12 +18,14 @@ namespace psl {
 
 enum StorageKind : int { kStoreF32 = 0, kStoreF16 = 1, kStoreBF16 = 2, kStoreF64 = 3 };
 
-// Read-only loads of the update kernels with a 256-byte L2 prefetch hint: a warp reads 64
-// (16-bit) or 128 (FP32) contiguous bytes of a row, and the warps of the next cells read
-// the rest of the same lines.
+// Loads of the update kernels with a 256-byte L2 prefetch hint: a warp reads 64 (16-bit) or
+// 128 (FP32) contiguous bytes of a row, and the warps of the next cells read the rest of the
+// same lines.  FP32: ordinary loads, since a dependent launch's blocks start before the kernel
+// ahead has written these values and load them after grid_wait, out of which their index comes
+// (psl_launch.cuh).  16-bit: the read-only path, in kernels launched the ordinary way.
 __device__ __forceinline__ float ldg_row(const float* p) {
   float v;
-  asm("ld.global.nc.L2::256B.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  asm("ld.global.L2::256B.f32 %0, [%1];" : "=f"(v) : "l"(p));
   return v;
 }
 __device__ __forceinline__ uint16_t ldg_row(const uint16_t* p) {
@@ -42,7 +44,7 @@ struct StoreF32 {
   __device__ __forceinline__ static void store(float* p, float v) { *p = v; }
   __device__ __forceinline__ static float load_q(const float* p, int) { return *p; }
   __device__ __forceinline__ static void store_q(float* p, float v, int) { *p = v; }
-  // Update-kernel forms: each element is read once by its owning cell (read-only path)
+  // Update-kernel forms: each element is read once by its owning cell
   // and then overwritten by it (evict-first store).
   template <int Q>
   __device__ __forceinline__ static float load_once(const float* p) { return ldg_row(p); }
@@ -103,7 +105,7 @@ struct StoreF64 {
   __device__ __forceinline__ static double load_q(const double* p, int) { return *p; }
   __device__ __forceinline__ static void store_q(double* p, double v, int) { *p = v; }
   template <int Q>
-  __device__ __forceinline__ static double load_once(const double* p) { return __ldg(p); }
+  __device__ __forceinline__ static double load_once(const double* p) { return *p; }
   template <int Q>
   __device__ __forceinline__ static void store_once(double* p, double v) { __stcs(p, v); }
 };

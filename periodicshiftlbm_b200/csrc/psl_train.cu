@@ -28,6 +28,7 @@
 #include "psl.h"
 #include "psl_internal.h"
 #include "psl_kernels.cuh"
+#include "psl_launch.cuh"
 #include "psl_mlp.cuh"
 
 using namespace psl;
@@ -82,11 +83,6 @@ struct GradTile {
 static_assert(sizeof(GradWeights) % 16 == 0 && sizeof(GradTile) % 16 == 0, "16-byte aligned rows");
 static_assert(sizeof(GradTile) >= (kTrainable + 1) * sizeof(float), "a warp's gradient fits its tile");
 constexpr size_t grad_smem(int warps) { return sizeof(GradWeights) + (size_t)warps * sizeof(GradTile); }
-
-// Programmatic dependent launch: a kernel's blocks may start before the kernel ahead of it in
-// the stream has finished; grid_wait returns once that one's writes are visible.
-__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 __device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 __device__ __forceinline__ void st4(float* p, float a, float b, float c, float d) {
@@ -576,38 +572,20 @@ struct psl_sgs_trainer {
 
 namespace {
 
-// A launch that may start while the kernel ahead of it in the stream is finishing (both
-// kernels wait for that one, grid_wait, before they touch anything it writes).
-template <typename... P, typename... A>
-cudaError_t launch_dependent(void (*kernel)(P...), unsigned int blocks, unsigned int threads, size_t smem, cudaStream_t stream,
-                             A... args) {
-  cudaLaunchAttribute attr{};
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(blocks);
-  cfg.blockDim = dim3(threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, args...);
-}
-
 // One warp per 32-sample tile while that many warps fit (14 per SM), so that a batch of 65,536
 // samples is one tile per warp on 148 x 14 warps and a small batch spreads over the SMs.
 int run_gradient(psl_sgs_trainer* t, long long first, long long count, int random, uint32_t seed, const AdamParams* adam) {
   const long long tiles = (count + kTile - 1) / kTile;
   const int blocks = (int)std::min<long long>(kGradBlocks, tiles);
   const int warps = (int)std::min<long long>(kMaxGradWarps, (tiles + blocks - 1) / blocks);
-  TRAIN_CUDA(launch_dependent(grad_kernel, blocks, 32 * warps, grad_smem(warps), t->stream, (const float*)t->params,
+  TRAIN_CUDA(launch_dependent(true, grad_kernel, dim3(blocks), 32 * warps, grad_smem(warps), t->stream, (const float*)t->params,
                               (const float*)t->X, (const float*)t->T, t->count, first, count, random, seed, t->partial));
   const unsigned int nb = (kTrainable + kReduceEntries) / kReduceEntries, threads = kReduceEntries * kReduceGroups;
   if (adam)
-    TRAIN_CUDA(launch_dependent(reduce_kernel<true>, nb, threads, 0, t->stream, (const float*)t->partial, blocks,
+    TRAIN_CUDA(launch_dependent(true, reduce_kernel<true>, dim3(nb), threads, 0, t->stream, (const float*)t->partial, blocks,
                                 count, t->grad, *adam));
   else
-    TRAIN_CUDA(launch_dependent(reduce_kernel<false>, nb, threads, 0, t->stream, (const float*)t->partial, blocks,
+    TRAIN_CUDA(launch_dependent(true, reduce_kernel<false>, dim3(nb), threads, 0, t->stream, (const float*)t->partial, blocks,
                                 count, t->grad, AdamParams{}));
   return PSL_OK;
 }
