@@ -476,11 +476,44 @@ __global__ void __launch_bounds__(kStepThreads) step_custom_kernel(const __grid_
 // ------------------------------------------------------------------------------------------
 // scalar transport (include/scalarTransportFunctions.h:10-176)
 // ------------------------------------------------------------------------------------------
+// The scalar populations of a block's cells, staged in shared memory (population-major, one
+// column per thread).  Each thread copies, reads and writes its own column only.
+constexpr int kScalarBlocks = 7;  // resident blocks per SM
+struct ScalarStage {
+  float T[27][kStepThreads];
+};
+// Starts the copy of the cell's 27 scalar populations into the thread's column
+// (cp.async: no registers hold them on the way); scalar_stage_wait before they are used.
+template <int Q = 0>
+__device__ __forceinline__ void scalar_stage_load(const RowIndex<StoreF32>& r, uint32_t cell, ScalarStage& st) {
+  if constexpr (Q < 27) {
+    uint32_t i = cell + r.off[Q];
+    if (cell >= r.lim[Q]) i -= r.n;
+    const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&st.T[Q][threadIdx.x]);
+    asm volatile("cp.async.ca.shared.global.L2::256B [%0], [%1], 4;" ::"r"(dst), "l"(r.base + i) : "memory");
+    scalar_stage_load<Q + 1>(r, cell, st);
+  }
+}
+// Population Q of the cell's scalar row.
+template <int Q>
+__device__ __forceinline__ void scalar_store(const RowIndex<StoreF32>& r, uint32_t cell, float v) {
+  uint32_t i = cell + r.off[Q];
+  if (cell >= r.lim[Q]) i -= r.n;
+  StoreF32::store_once<Q>(r.base + i, v);
+}
+__device__ __forceinline__ void scalar_stage_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // Collision of the scalar populations T_q after the flow collision, after Zhang, Fan & Chen
 // (2011, eqs 2.5-2.7) as applyScalarTransportCollision uses them: with the post-collision
 // populations f, T_mean = sum f T / rho, S = sum c (f (T - T_mean)),
 // F_q = 3/rho (c_q - u) . S and T_q <- T_mean + (1 - 1/tau_T) F_q.  sum f T is unchanged.
-__device__ __forceinline__ void scalar_collision(const float (&f)[27], float (&T)[27], float tauT) {
+// T comes from the thread's staged column, or is `given` everywhere when `prescribed`; the
+// new T_q depends on f only through the sums here.
+struct ScalarSums {
+  float tm, ux, uy, uz, sx, sy, sz, a;
+};
+__device__ __forceinline__ ScalarSums scalar_sums(const float (&f)[27], const ScalarStage& st, bool prescribed, float given,
+                                                  float tauT) {
   float rho = 0.f, jx = 0.f, jy = 0.f, jz = 0.f, ft = 0.f;
 #pragma unroll
   for (int q = 0; q < 27; ++q) {
@@ -488,22 +521,31 @@ __device__ __forceinline__ void scalar_collision(const float (&f)[27], float (&T
     jx += cx(q) * f[q];
     jy += cy(q) * f[q];
     jz += cz(q) * f[q];
-    ft += f[q] * T[q];
+    ft += f[q] * (prescribed ? given : st.T[q][threadIdx.x]);
   }
   const float inv_rho = 1.f / rho;
-  const float ux = jx * inv_rho, uy = jy * inv_rho, uz = jz * inv_rho;
-  const float tm = ft * inv_rho;
-  float sx = 0.f, sy = 0.f, sz = 0.f;
+  ScalarSums r;
+  r.ux = jx * inv_rho;
+  r.uy = jy * inv_rho;
+  r.uz = jz * inv_rho;
+  r.tm = ft * inv_rho;
+  r.sx = r.sy = r.sz = 0.f;
 #pragma unroll
   for (int q = 0; q < 27; ++q) {
-    const float g = f[q] * (T[q] - tm);
-    sx += cx(q) * g;
-    sy += cy(q) * g;
-    sz += cz(q) * g;
+    const float g = f[q] * ((prescribed ? given : st.T[q][threadIdx.x]) - r.tm);
+    r.sx += cx(q) * g;
+    r.sy += cy(q) * g;
+    r.sz += cz(q) * g;
   }
-  const float a = (1.f - 1.f / tauT) * 3.f * inv_rho;
-#pragma unroll
-  for (int q = 0; q < 27; ++q) T[q] = tm + a * ((cx(q) - ux) * sx + (cy(q) - uy) * sy + (cz(q) - uz) * sz);
+  r.a = (1.f - 1.f / tauT) * 3.f * inv_rho;
+  return r;
+}
+template <int Q = 0>
+__device__ __forceinline__ void scalar_rebuild_store(const RowIndex<StoreF32>& r, uint32_t cell, const ScalarSums& c) {
+  if constexpr (Q < 27) {
+    scalar_store<Q>(r, cell, c.tm + c.a * ((cx(Q) - c.ux) * c.sx + (cy(Q) - c.uy) * c.sy + (cz(Q) - c.uz) * c.sz));
+    scalar_rebuild_store<Q + 1>(r, cell, c);
+  }
 }
 
 template <typename S>
@@ -517,47 +559,72 @@ struct ScalarParams {
 // applyLocalCellUpdate with scalar transport (scalarTransportFunctions.h:10-107): T is
 // bounced back with f in solid cells, mirrored with f in free-slip cells, set to the given
 // concentration where one is prescribed, and collided after the flow collision.
+//
+// What bounds it: HBM, 432 bytes per cell in FP32.  T is not needed before the flow has
+// collided, so it waits in shared memory (13.8 KB per block) instead of 27 registers: with
+// both sets in registers the kernel held 96 of them and 20 warps per SM, 171.7 us for
+// 192x98x96 cells; now 72 registers and 28 warps, and the whole step with its periodic copy
+// went from 200 to 161 us.  (Two stages of 13.8 KB and the 1 KB each block reserves allow 7
+// blocks per SM; capping the registers at 64 for an eighth gained nothing.)
 template <typename S>
-__global__ void __launch_bounds__(kStepThreads) step_scalar_kernel(const __grid_constant__ ScalarParams<S> sp) {
+__global__ void __launch_bounds__(kStepThreads, kScalarBlocks) step_scalar_kernel(const __grid_constant__ ScalarParams<S> sp) {
+  __shared__ ScalarStage st;
+  __shared__ float slot[kStepThreads][27];
   const StepParams<S>& p = sp.base;
   const uint32_t cell = blockIdx.x * kStepThreads + threadIdx.x;
   if (cell >= p.ri.n) return;
   const uint8_t m = p.marker[cell];
   const int kind = marker_kind(m);
   if (kind == kSkip) return;
-  float f[27], T[27];
+  float f[27];
   load_cell_ri<S>(p.ri, cell, f);
-  load_cell_ri<StoreF32>(sp.T, cell, T);
+  scalar_stage_load(sp.T, cell, st);
   if (kind == kSolid) {
 #pragma unroll
     for (int q = 1; q < 27; q += 2) {
-      const float a = f[q], b = T[q];
+      const float a = f[q];
       f[q] = f[q + 1];
       f[q + 1] = a;
-      T[q] = T[q + 1];
-      T[q + 1] = b;
+    }
+    store_cell_ri<S>(p.ri, cell, f);
+    scalar_stage_wait();
+    // a rolled loop: unrolled, its addresses were held from the loads on and spilled
+#pragma unroll 1
+    for (int q = 0; q < 27; ++q) {
+      uint32_t i = cell + sp.T.off[q];
+      if (cell >= sp.T.lim[q]) i -= sp.T.n;
+      __stcs(sp.T.base + i, st.T[q == 0 ? 0 : (q & 1) ? q + 1 : q - 1][threadIdx.x]);
     }
   } else {
-    if (kind != kFluid) {
-      apply_boundary(m, f, p.given ? p.given[cell] : p.given_uniform);
-      if (kind == kMirror) bc::mirror(marker_normal(m), T);
-    }
-    if (sp.givenT) {
-      const float tg = sp.givenT[cell];
-      if (tg == tg) {
+    if (kind != kFluid) {  // f waits in the thread's boundary slot while T is mirrored
+      float* mine = slot[threadIdx.x];
 #pragma unroll
-        for (int q = 0; q < 27; ++q) T[q] = tg;
+      for (int q = 0; q < 27; ++q) mine[q] = f[q];
+      apply_boundary_out_of_line(m, mine, p.given ? p.given[cell] : p.given_uniform);
+      if (kind == kMirror) {
+        float T[27];
+        scalar_stage_wait();
+#pragma unroll
+        for (int q = 0; q < 27; ++q) T[q] = st.T[q][threadIdx.x];
+        bc::mirror(marker_normal(m), T);
+#pragma unroll
+        for (int q = 0; q < 27; ++q) st.T[q][threadIdx.x] = T[q];
       }
+#pragma unroll
+      for (int q = 0; q < 27; ++q) f[q] = mine[q];
     }
+    float tg = __int_as_float(0x7fffffff);  // NaN: none prescribed
+    if (sp.givenT) tg = sp.givenT[cell];
     collide<false>(f, cell_relaxation(p.rx, p.cs, cell));
-    scalar_collision(f, T, sp.tauT);
     if (p.health) {
       const float r = f[0] + f[1] + f[2] + f[3] + f[4] + f[5] + f[6];
       if (!(r > 0.f && r < 1.0e30f)) atomicOr(p.health, 1u);
     }
+    scalar_stage_wait();
+    const ScalarSums c = scalar_sums(f, st, tg == tg, tg, sp.tauT);
+    store_cell_ri<S>(p.ri, cell, f);
+    scalar_rebuild_store(sp.T, cell, c);
   }
-  store_cell_ri<S>(p.ri, cell, f);
-  store_cell_ri<StoreF32>(sp.T, cell, T);
 }
 
 // Per-cell concentration sum f T / rho (FP64 sums) in logical order.
