@@ -200,6 +200,7 @@ int psl_grid_destroy(psl_grid* g) {
   if (g->given) cudaFree(g->given);
   if (g->health) cudaFree(g->health);
   if (g->scratch) cudaFree(g->scratch);
+  if (g->stage) cudaFree(g->stage);
   if (g->mlp) cudaFree(g->mlp);
   if (g->T) cudaFree(g->T);
   if (g->givenT) cudaFree(g->givenT);
@@ -358,27 +359,9 @@ int psl_set_scalar_given_field(psl_grid* g, const float* host) {
   return PSL_OK;
 }
 
+static cudaError_t copy_rows_f32(psl_grid* g, float* base, size_t row_stride, bool twice, float* host, bool to_host);
 static int scalar_rows(psl_grid* g, float* host, bool get) {
-  float* tmp = nullptr;
-  PSL_CUDA(cudaMalloc(&tmp, (size_t)g->n * sizeof(float)));
-  cudaError_t e = cudaStreamSynchronize(g->stream);
-  const GridView<StoreF32> v = scalar_view(g);
-  for (int q = 0; q < 27 && e == cudaSuccess; ++q) {
-    if (get) {
-      gather_logical_kernel<StoreF32><<<blocks_for(g->n, 256), 256, 0, g->stream>>>(v, q, tmp);
-      e = cudaGetLastError();
-      if (e == cudaSuccess)
-        e = cudaMemcpyAsync(host + (size_t)q * g->n, tmp, (size_t)g->n * sizeof(float), cudaMemcpyDeviceToHost, g->stream);
-    } else {
-      e = cudaMemcpyAsync(tmp, host + (size_t)q * g->n, (size_t)g->n * sizeof(float), cudaMemcpyHostToDevice, g->stream);
-      if (e == cudaSuccess) {
-        scatter_logical_kernel<StoreF32><<<blocks_for(g->n, 256), 256, 0, g->stream>>>(v, q, tmp);
-        e = cudaGetLastError();
-      }
-    }
-  }
-  if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
-  cudaFree(tmp);
+  const cudaError_t e = copy_rows_f32(g, g->T, g->stride, false, host, get);
   if (e != cudaSuccess) return fail(PSL_ERR_CUDA, std::string("psl scalar populations: ") + cudaGetErrorString(e));
   return PSL_OK;
 }
@@ -953,18 +936,17 @@ int psl_sphere_force_async(psl_grid* g, const psl_sphere_case* sc, double* force
 }
 
 // ---- data movement ----
-// FP32 storage needs no conversion: logical row q is the stored row rotated by shift_q
+// FP32 rows need no conversion: logical row q is the stored row rotated by shift_q
 // (cell c at (c + shift_q) mod N), so it moves with plain copies -- one contiguous range on
 // twice-mapped rows (the second mapping holds the wrap), else the two pieces of the
 // rotation -- without a staging buffer or a kernel.
-static cudaError_t copy_rows_f32(psl_grid* g, float* host, bool to_host) {
-  float* base = static_cast<float*>(g->f);
+static cudaError_t copy_rows_f32(psl_grid* g, float* base, size_t row_stride, bool twice, float* host, bool to_host) {
   const size_t n = g->n;
   for (int q = 0; q < 27; ++q) {
-    float* row = base + (size_t)q * g->f_stride;
+    float* row = base + (size_t)q * row_stride;
     float* h = host + (size_t)q * n;
     const size_t sh = g->shift[q];
-    const size_t first = g->f_twice ? n : n - sh;  // elements of the first piece
+    const size_t first = twice ? n : n - sh;  // elements of the first piece
     cudaError_t e = to_host ? cudaMemcpyAsync(h, row + sh, first * sizeof(float), cudaMemcpyDeviceToHost, g->stream)
                             : cudaMemcpyAsync(row + sh, h, first * sizeof(float), cudaMemcpyHostToDevice, g->stream);
     if (e == cudaSuccess && first < n)
@@ -975,16 +957,27 @@ static cudaError_t copy_rows_f32(psl_grid* g, float* host, bool to_host) {
   return cudaStreamSynchronize(g->stream);
 }
 
+// The grid's staging row for converting reads and writes, N floats, made on first use and kept
+// until the grid is destroyed: allocated and freed in every call it cost more than the
+// conversion, and now and then many times the whole read (251x117x125 BF16 grid: 9-95 ms per
+// read of 396 MB).
+static cudaError_t staging_row(psl_grid* g, float** out) {
+  cudaError_t e = cudaSuccess;
+  if (!g->stage) e = cudaMalloc(&g->stage, (size_t)g->n * sizeof(float));
+  if (e != cudaSuccess) g->stage = nullptr;
+  *out = g->stage;
+  return e;
+}
+
 template <typename S>
 static int gather(psl_grid* g, float* host) {
   if constexpr (S::kind == kStoreF32) {
-    const cudaError_t e = copy_rows_f32(g, host, true);
+    const cudaError_t e = copy_rows_f32(g, static_cast<float*>(g->f), g->f_stride, g->f_twice, host, true);
     if (e != cudaSuccess) return fail(PSL_ERR_CUDA, std::string("psl_get_populations: ") + cudaGetErrorString(e));
     return PSL_OK;
   }
   float* tmp = nullptr;
-  PSL_CUDA(cudaMalloc(&tmp, (size_t)g->n * sizeof(float)));
-  cudaError_t e = cudaSuccess;
+  cudaError_t e = staging_row(g, &tmp);
   const GridView<S> v = view<S>(g);
   // one staging row; stream order serialises each row's gather after the previous copy
   for (int q = 0; q < 27 && e == cudaSuccess; ++q) {
@@ -994,21 +987,23 @@ static int gather(psl_grid* g, float* host) {
       e = cudaMemcpyAsync(host + (size_t)q * g->n, tmp, (size_t)g->n * sizeof(float), cudaMemcpyDeviceToHost, g->stream);
   }
   if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
-  cudaFree(tmp);
-  if (e != cudaSuccess) return fail(PSL_ERR_CUDA, std::string("psl_get_populations: ") + cudaGetErrorString(e));
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return fail(PSL_ERR_CUDA, std::string("psl_get_populations: ") + cudaGetErrorString(e));
+  }
   return PSL_OK;
 }
 
 template <typename S>
 static int scatter(psl_grid* g, const float* host) {
   if constexpr (S::kind == kStoreF32) {
-    const cudaError_t e = copy_rows_f32(g, const_cast<float*>(host), false);
+    const cudaError_t e =
+        copy_rows_f32(g, static_cast<float*>(g->f), g->f_stride, g->f_twice, const_cast<float*>(host), false);
     if (e != cudaSuccess) return fail(PSL_ERR_CUDA, std::string("psl_set_populations: ") + cudaGetErrorString(e));
     return PSL_OK;
   }
   float* tmp = nullptr;
-  PSL_CUDA(cudaMalloc(&tmp, (size_t)g->n * sizeof(float)));
-  cudaError_t e = cudaSuccess;
+  cudaError_t e = staging_row(g, &tmp);
   const GridView<S> v = view<S>(g);
   for (int q = 0; q < 27 && e == cudaSuccess; ++q) {
     e = cudaMemcpyAsync(tmp, host + (size_t)q * g->n, (size_t)g->n * sizeof(float), cudaMemcpyHostToDevice, g->stream);
@@ -1018,8 +1013,10 @@ static int scatter(psl_grid* g, const float* host) {
     }
   }
   if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
-  cudaFree(tmp);
-  if (e != cudaSuccess) return fail(PSL_ERR_CUDA, std::string("psl_set_populations: ") + cudaGetErrorString(e));
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return fail(PSL_ERR_CUDA, std::string("psl_set_populations: ") + cudaGetErrorString(e));
+  }
   return PSL_OK;
 }
 
