@@ -1004,7 +1004,7 @@ __device__ __forceinline__ void force_partial(const GridView<S>& g, const uint8_
     const int i = i0 + (int)(t % si), j = j0 + (int)((t / si) % sj), k = k0 + (int)(t / (si * sj));
     const uint32_t cell = ((uint32_t)k * ny + j) * nx + i;
     if (marker_kind(marker[cell]) != kSolid) continue;
-    double rho = 0, jx = 0, jy = 0, jz = 0, bx = 0, by = 0, bz = 0;
+    double rho = 0, jx = 0, jy = 0, jz = 0;
 #pragma unroll
     for (int q = 0; q < 27; ++q) {
       const double v = (double)S::load_q(g.fq[q] + shifted(cell, g.shift[q], g.n), q);
@@ -1012,14 +1012,12 @@ __device__ __forceinline__ void force_partial(const GridView<S>& g, const uint8_
       jx += cx(q) * v;
       jy += cy(q) * v;
       jz += cz(q) * v;
-      // the bounced population of direction q sits in direction opposite(q)
-      bx -= cx(q) * v;
-      by -= cy(q) * v;
-      bz -= cz(q) * v;
     }
-    acc[0] += rho * (jx / rho - bx / rho);
-    acc[1] += rho * (jy / rho - by / rho);
-    acc[2] += rho * (jz / rho - bz / rho);
+    // rho (u - u_bounced): the bounced population of direction q sits in direction opposite(q),
+    // so the bounced momentum is -j to the last bit and the difference 2 j / rho
+    acc[0] += rho * (2.0 * (jx / rho));
+    acc[1] += rho * (2.0 * (jy / rho));
+    acc[2] += rho * (2.0 * (jz / rho));
   }
   __shared__ double red[3][kForceThreads];
   for (int c = 0; c < 3; ++c) red[c][threadIdx.x] = acc[c];
