@@ -524,6 +524,8 @@ static cudaError_t launch_step(psl_grid* g, bool held_nu, const ThreadRange& ran
   p.rx = relaxation<typename S::calc>(g);
   p.health = g->health;
   p.ri = row_index<S>(g);
+  p.flat.base = p.ri.base;
+  for (int q = 0; q < 27; ++q) p.flat.byte_off[q] = (uint64_t)p.ri.off[q] * sizeof(typename S::type);
   p.rot = thread_rotation(g);
   p.nut = g->mlp_nut;
   p.nu = g->info.nu;

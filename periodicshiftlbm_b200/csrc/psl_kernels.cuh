@@ -51,6 +51,16 @@ struct RowIndex {
   uint32_t n;
 };
 
+// Byte offset of population q's element of cell 0: an address is one 64-bit addition to the
+// cell's own byte address, where base + (cell + off_q) takes a 32-bit addition and a widening
+// multiply-add.  On rows mapped twice: 128x64x64 sphere with its drag 29.9 -> 28.7 us per step,
+// refined 256x128x128 FP16 sphere 233.1 -> 229.4 us, refined 512x256x256 FP16 with the closure
+// 1.732 -> 1.688 ms.
+template <typename S>
+struct FlatIndex {
+  typename S::type* base;
+  uint64_t byte_off[27];
+};
 
 // The threads of an update launch: launch thread u (u < count) is thread
 // t_begin + u + (u >= gap_at ? gap_len : 0) of cell_of_thread, so one launch can run a
@@ -67,6 +77,7 @@ template <typename S>
 struct StepParams {
   GridView<S> g;
   RowIndex<S> ri;
+  FlatIndex<S> flat;     // kAddrFlat, and kAddrIndex in FP32
   const uint8_t* marker;
   const float4* given;   // per-cell (rho, ux, uy, uz) for boundary cells, or null
   float4 given_uniform;  // used when `given` is null
@@ -204,19 +215,60 @@ __device__ __forceinline__ void store_cell(const GridView<S>& g, uint32_t cell, 
 }
 // Rows mapped twice (psl_rowmap.cu): cell + off_q < row start + 2N addresses the wrapped
 // element through the row's second mapping, so no wrap compare.
-template <typename A, typename S, int Q = 0>
-__device__ __forceinline__ void load_cell_flat(const RowIndex<S>& r, uint32_t cell, typename A::calc (&f)[27]) {
+template <typename A, int Q = 0, typename E>
+__device__ __forceinline__ void load_flat_from(const E* at, const uint64_t (&off)[27], typename A::calc (&f)[27]) {
   if constexpr (Q < 27) {
-    f[Q] = A::template load_once<Q>(r.base + (cell + r.off[Q]));
-    load_cell_flat<A, S, Q + 1>(r, cell, f);
+    f[Q] = A::template load_once<Q>(reinterpret_cast<const E*>(reinterpret_cast<const char*>(at) + off[Q]));
+    load_flat_from<A, Q + 1>(at, off, f);
   }
 }
-template <typename A, typename S, int Q = 0>
-__device__ __forceinline__ void store_cell_flat(const RowIndex<S>& r, uint32_t cell, const typename A::calc (&f)[27]) {
+template <typename A, int Q = 0, typename E>
+__device__ __forceinline__ void store_flat_from(E* at, const uint64_t (&off)[27], const typename A::calc (&f)[27]) {
   if constexpr (Q < 27) {
-    A::template store_once<Q>(r.base + (cell + r.off[Q]), f[Q]);
-    store_cell_flat<A, S, Q + 1>(r, cell, f);
+    A::template store_once<Q>(reinterpret_cast<E*>(reinterpret_cast<char*>(at) + off[Q]), f[Q]);
+    store_flat_from<A, Q + 1>(at, off, f);
   }
+}
+// The same with the periodic wrap: the element N lower where the cell is past the row's limit.
+// FP32 only (257x257x256 box 696 -> 684 us per step): the 16-bit kernels spill at their register
+// cap (251x117x125 BF16 grid 127.2 -> 131.3 us).
+template <typename A, int Q = 0, typename E>
+__device__ __forceinline__ void load_wrap_from(const E* at, uint32_t cell, const uint64_t (&off)[27], const uint32_t (&lim)[27],
+                                               uint32_t n, typename A::calc (&f)[27]) {
+  if constexpr (Q < 27) {
+    const char* a = reinterpret_cast<const char*>(at) + off[Q];
+    if (cell >= lim[Q]) a -= (uint64_t)n * sizeof(E);
+    f[Q] = A::template load_once<Q>(reinterpret_cast<const E*>(a));
+    load_wrap_from<A, Q + 1>(at, cell, off, lim, n, f);
+  }
+}
+template <typename A, int Q = 0, typename E>
+__device__ __forceinline__ void store_wrap_from(E* at, uint32_t cell, const uint64_t (&off)[27], const uint32_t (&lim)[27],
+                                                uint32_t n, const typename A::calc (&f)[27]) {
+  if constexpr (Q < 27) {
+    char* a = reinterpret_cast<char*>(at) + off[Q];
+    if (cell >= lim[Q]) a -= (uint64_t)n * sizeof(E);
+    A::template store_once<Q>(reinterpret_cast<E*>(a), f[Q]);
+    store_wrap_from<A, Q + 1>(at, cell, off, lim, n, f);
+  }
+}
+template <typename A, typename S>
+__device__ __forceinline__ void load_cell_wrap(const FlatIndex<S>& r, const RowIndex<S>& ri, uint32_t cell,
+                                               typename A::calc (&f)[27]) {
+  load_wrap_from<A>(static_cast<const typename S::type*>(r.base + cell), cell, r.byte_off, ri.lim, ri.n, f);
+}
+template <typename A, typename S>
+__device__ __forceinline__ void store_cell_wrap(const FlatIndex<S>& r, const RowIndex<S>& ri, uint32_t cell,
+                                                const typename A::calc (&f)[27]) {
+  store_wrap_from<A>(r.base + cell, cell, r.byte_off, ri.lim, ri.n, f);
+}
+template <typename A, typename S>
+__device__ __forceinline__ void load_cell_flat(const FlatIndex<S>& r, uint32_t cell, typename A::calc (&f)[27]) {
+  load_flat_from<A>(static_cast<const typename S::type*>(r.base + cell), r.byte_off, f);
+}
+template <typename A, typename S>
+__device__ __forceinline__ void store_cell_flat(const FlatIndex<S>& r, uint32_t cell, const typename A::calc (&f)[27]) {
+  store_flat_from<A>(r.base + cell, r.byte_off, f);
 }
 template <typename S>
 __device__ __forceinline__ void load_cell_ri(const RowIndex<S>& r, uint32_t cell, typename S::calc (&f)[27]) {
@@ -258,13 +310,15 @@ enum RowAddr : int { kAddrView = 0, kAddrIndex = 1, kAddrFlat = 2 };
 
 template <typename A, int kAddr, typename S>
 __device__ __forceinline__ void load_for(const StepParams<S>& p, uint32_t cell, typename A::calc (&f)[27]) {
-  if constexpr (kAddr == kAddrFlat) load_cell_flat<A>(p.ri, cell, f);
+  if constexpr (kAddr == kAddrFlat) load_cell_flat<A>(p.flat, cell, f);
+  else if constexpr (kAddr == kAddrIndex && S::kind == kStoreF32) load_cell_wrap<A>(p.flat, p.ri, cell, f);
   else if constexpr (kAddr == kAddrIndex) load_cell_as<A>(p.ri, cell, f);
   else load_cell_as<A>(p.g, cell, f);
 }
 template <typename A, int kAddr, typename S>
 __device__ __forceinline__ void store_for(const StepParams<S>& p, uint32_t cell, const typename A::calc (&f)[27]) {
-  if constexpr (kAddr == kAddrFlat) store_cell_flat<A>(p.ri, cell, f);
+  if constexpr (kAddr == kAddrFlat) store_cell_flat<A>(p.flat, cell, f);
+  else if constexpr (kAddr == kAddrIndex && S::kind == kStoreF32) store_cell_wrap<A>(p.flat, p.ri, cell, f);
   else if constexpr (kAddr == kAddrIndex) store_cell_as<A>(p.ri, cell, f);
   else store_cell_as<A>(p.g, cell, f);
 }

@@ -114,7 +114,9 @@ int launch(psl_grid* g, const ThreadRange& range) {
   for (int q = 0; q < 27; ++q) {
     p.ri.off[q] = (uint32_t)((size_t)q * g->f_stride + g->shift[q]);
     p.ri.lim[q] = g->n - g->shift[q];
+    p.flat.byte_off[q] = (uint64_t)p.ri.off[q] * sizeof(typename S::type);
   }
+  p.flat.base = p.ri.base;
   p.marker = g->marker;
   p.given = g->given;
   p.given_uniform = g->given_uniform;

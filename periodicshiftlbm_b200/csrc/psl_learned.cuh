@@ -22,6 +22,7 @@ namespace psl {
 template <typename S>
 struct LearnedParams {
   RowIndex<S> ri;
+  FlatIndex<S> flat;         // kFlat
   const uint8_t* marker;
   const float4* given;
   float4 given_uniform;
@@ -64,14 +65,14 @@ __device__ __forceinline__ void mlp_features_d(const CellMomentsG& m, float widt
 // moment sums from the stored bits; FP32 runs the plain FP32 update's operation order, only
 // the rate differs.  kFlat: rows mapped twice, addressed without the wrap.
 template <typename A, bool kFlat, typename S>
-__device__ __forceinline__ void load_rows(const RowIndex<S>& r, uint32_t cell, typename A::calc (&f)[27]) {
-  if constexpr (kFlat) load_cell_flat<A>(r, cell, f);
-  else load_cell_as<A>(r, cell, f);
+__device__ __forceinline__ void load_rows(const LearnedParams<S>& p, uint32_t cell, typename A::calc (&f)[27]) {
+  if constexpr (kFlat) load_cell_flat<A>(p.flat, cell, f);
+  else load_cell_as<A>(p.ri, cell, f);
 }
 template <typename A, bool kFlat, typename S>
-__device__ __forceinline__ void store_rows(const RowIndex<S>& r, uint32_t cell, const typename A::calc (&f)[27]) {
-  if constexpr (kFlat) store_cell_flat<A>(r, cell, f);
-  else store_cell_as<A>(r, cell, f);
+__device__ __forceinline__ void store_rows(const LearnedParams<S>& p, uint32_t cell, const typename A::calc (&f)[27]) {
+  if constexpr (kFlat) store_cell_flat<A>(p.flat, cell, f);
+  else store_cell_as<A>(p.ri, cell, f);
 }
 
 // 7 blocks of 128 per SM (72 registers; ptxas keeps ~40 bytes in local memory, L1-resident):
@@ -95,16 +96,16 @@ __global__ void __launch_bounds__(kStepThreads, 7) step_learned_warp_kernel(cons
     using B = StoredBits<S>;
     uint16_t h[27];
     if (kind == kSolid) {  // bounce-back: done before the closure, nothing to keep
-      load_rows<B, kFlat>(p.ri, cell, h);
+      load_rows<B, kFlat>(p, cell, h);
 #pragma unroll
       for (int q = 1; q < 27; q += 2) {
         const uint16_t t = h[q];
         h[q] = h[q + 1];
         h[q + 1] = t;
       }
-      store_rows<B, kFlat>(p.ri, cell, h);
+      store_rows<B, kFlat>(p, cell, h);
     }
-    if (collides) load_rows<B, kFlat>(p.ri, cell, h);
+    if (collides) load_rows<B, kFlat>(p, cell, h);
     CellMomentsG cm{};
     const bool bc = collides && kind != kFluid;
     if (!__any_sync(0xffffffffu, bc)) {
@@ -132,21 +133,21 @@ __global__ void __launch_bounds__(kStepThreads, 7) step_learned_warp_kernel(cons
     if (collides) {
       if constexpr (kStoreNu) p.nut[cell] = __half_as_ushort(__float2half_rn(nu_t));
       relax_rebuild_g(f, cm, grecip(3.f * (p.nu + nu_t) + 0.5f));
-      store_rows<StoredOf<S>, kFlat>(p.ri, cell, f);
+      store_rows<StoredOf<S>, kFlat>(p, cell, f);
     }
   } else {
     using A = StoredOf<S>;
     if (kind == kSolid) {  // bounce-back: done before the closure, nothing to keep
-      load_rows<A, kFlat>(p.ri, cell, f);
+      load_rows<A, kFlat>(p, cell, f);
 #pragma unroll
       for (int q = 1; q < 27; q += 2) {
         const float t = f[q];
         f[q] = f[q + 1];
         f[q + 1] = t;
       }
-      store_rows<A, kFlat>(p.ri, cell, f);
+      store_rows<A, kFlat>(p, cell, f);
     }
-    if (collides) load_rows<A, kFlat>(p.ri, cell, f);
+    if (collides) load_rows<A, kFlat>(p, cell, f);
     float K[3][3][3];
     float rho = 1.f, ux = 0.f, uy = 0.f, uz = 0.f, inv_rho = 1.f;
     if (collides) {
@@ -162,7 +163,7 @@ __global__ void __launch_bounds__(kStepThreads, 7) step_learned_warp_kernel(cons
         const float r = f[0] + f[1] + f[2] + f[3] + f[4] + f[5] + f[6];
         if (!(r > 0.f && r < 1.0e30f)) atomicOr(p.health, 1u);
       }
-      store_rows<A, kFlat>(p.ri, cell, f);
+      store_rows<A, kFlat>(p, cell, f);
     }
   }
 }
