@@ -200,7 +200,6 @@ int psl_grid_destroy(psl_grid* g) {
   if (g->given) cudaFree(g->given);
   if (g->health) cudaFree(g->health);
   if (g->scratch) cudaFree(g->scratch);
-  if (g->stage) cudaFree(g->stage);
   if (g->mlp) cudaFree(g->mlp);
   if (g->T) cudaFree(g->T);
   if (g->givenT) cudaFree(g->givenT);
@@ -959,18 +958,6 @@ static cudaError_t copy_rows_f32(psl_grid* g, float* base, size_t row_stride, bo
   return cudaStreamSynchronize(g->stream);
 }
 
-// The grid's staging row for converting reads and writes, N floats, made on first use and kept
-// until the grid is destroyed: allocated and freed in every call it cost more than the
-// conversion, and now and then many times the whole read (251x117x125 BF16 grid: 9-95 ms per
-// read of 396 MB).
-static cudaError_t staging_row(psl_grid* g, float** out) {
-  cudaError_t e = cudaSuccess;
-  if (!g->stage) e = cudaMalloc(&g->stage, (size_t)g->n * sizeof(float));
-  if (e != cudaSuccess) g->stage = nullptr;
-  *out = g->stage;
-  return e;
-}
-
 template <typename S>
 static int gather(psl_grid* g, float* host) {
   if constexpr (S::kind == kStoreF32) {
@@ -979,7 +966,8 @@ static int gather(psl_grid* g, float* host) {
     return PSL_OK;
   }
   float* tmp = nullptr;
-  cudaError_t e = staging_row(g, &tmp);
+  PSL_CUDA(cudaMalloc(&tmp, (size_t)g->n * sizeof(float)));
+  cudaError_t e = cudaSuccess;
   const GridView<S> v = view<S>(g);
   // one staging row; stream order serialises each row's gather after the previous copy
   for (int q = 0; q < 27 && e == cudaSuccess; ++q) {
@@ -989,10 +977,8 @@ static int gather(psl_grid* g, float* host) {
       e = cudaMemcpyAsync(host + (size_t)q * g->n, tmp, (size_t)g->n * sizeof(float), cudaMemcpyDeviceToHost, g->stream);
   }
   if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
-  if (e != cudaSuccess) {
-    cudaGetLastError();
-    return fail(PSL_ERR_CUDA, std::string("psl_get_populations: ") + cudaGetErrorString(e));
-  }
+  cudaFree(tmp);
+  if (e != cudaSuccess) return fail(PSL_ERR_CUDA, std::string("psl_get_populations: ") + cudaGetErrorString(e));
   return PSL_OK;
 }
 
@@ -1005,7 +991,8 @@ static int scatter(psl_grid* g, const float* host) {
     return PSL_OK;
   }
   float* tmp = nullptr;
-  cudaError_t e = staging_row(g, &tmp);
+  PSL_CUDA(cudaMalloc(&tmp, (size_t)g->n * sizeof(float)));
+  cudaError_t e = cudaSuccess;
   const GridView<S> v = view<S>(g);
   for (int q = 0; q < 27 && e == cudaSuccess; ++q) {
     e = cudaMemcpyAsync(tmp, host + (size_t)q * g->n, (size_t)g->n * sizeof(float), cudaMemcpyHostToDevice, g->stream);
@@ -1015,10 +1002,8 @@ static int scatter(psl_grid* g, const float* host) {
     }
   }
   if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
-  if (e != cudaSuccess) {
-    cudaGetLastError();
-    return fail(PSL_ERR_CUDA, std::string("psl_set_populations: ") + cudaGetErrorString(e));
-  }
+  cudaFree(tmp);
+  if (e != cudaSuccess) return fail(PSL_ERR_CUDA, std::string("psl_set_populations: ") + cudaGetErrorString(e));
   return PSL_OK;
 }
 
