@@ -1,5 +1,6 @@
 // C ABI of the lattice update (include/psl.h): grid handles, set-up, per-step launches,
 // reductions and data movement.  Host-side logic only; the kernels are in psl_kernels.cuh.
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -13,6 +14,7 @@
 #include <vector>
 
 #include "psl.h"
+#include "psl_destination.h"
 #include "psl_internal.h"
 #include "psl_kernels.cuh"
 #include "psl_launch.cuh"
@@ -907,18 +909,49 @@ int psl_sphere_force(psl_grid* g, const psl_sphere_case* sc, double* force3) {
   return PSL_OK;
 }
 
-// The address at which a kernel on `device` can write the three doubles at p: p in that
-// device's memory, managed memory or pinned host memory mapped into it; null when p has to be
-// reached by a copy (another device's memory, pageable memory, a misaligned address).
-static double* device_writable(double* p, int device) {
-  if (reinterpret_cast<uintptr_t>(p) % alignof(double) != 0) return nullptr;
+// What the driver reports about p; all zero where it cannot tell.
+static PointerFacts pointer_facts(const void* p) {
+  static const auto attributes = [] {  // the library does not link libcuda
+    void* fn = nullptr;
+    cudaDriverEntryPointQueryResult found = cudaDriverEntryPointSymbolNotFound;
+    if (cudaGetDriverEntryPoint("cuPointerGetAttributes", &fn, cudaEnableDefault, &found) != cudaSuccess ||
+        found != cudaDriverEntryPointSuccess) {
+      cudaGetLastError();
+      fn = nullptr;
+    }
+    return reinterpret_cast<decltype(&cuPointerGetAttributes)>(fn);
+  }();
+  PointerFacts f;
   cudaPointerAttributes a{};
   if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
     cudaGetLastError();
-    return nullptr;
+    return f;
   }
-  if (a.type == cudaMemoryTypeUnregistered || (a.type == cudaMemoryTypeDevice && a.device != device)) return nullptr;
-  return static_cast<double*>(a.devicePointer);
+  if (a.type == cudaMemoryTypeUnregistered) return f;  // pageable memory
+  f.device_memory = a.type == cudaMemoryTypeDevice;
+  f.device = a.device;
+  f.mapped = reinterpret_cast<uint64_t>(a.devicePointer);
+  CUdeviceptr start = 0;
+  size_t size = 0;
+  unsigned long long access = 0;
+  CUpointer_attribute what[3] = {CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE,
+                                 CU_POINTER_ATTRIBUTE_ACCESS_FLAGS};
+  void* into[3] = {&start, &size, &access};
+  if (attributes && attributes(3, what, into, reinterpret_cast<CUdeviceptr>(p)) == CUDA_SUCCESS) {
+    f.range_start = start;
+    f.range_size = size;
+    f.access = (unsigned int)access;
+  }
+  return f;
+}
+
+// The address at which a kernel on `device` can write the three doubles at p, or null when they
+// have to be reached by a copy.
+static double* device_writable(double* p, int device) {
+  const PointerFacts f = pointer_facts(p);
+  return kernel_may_write(f, reinterpret_cast<uint64_t>(p), 3 * sizeof(double), alignof(double), device)
+             ? reinterpret_cast<double*>(f.mapped)
+             : nullptr;
 }
 
 int psl_sphere_force_async(psl_grid* g, const psl_sphere_case* sc, double* force3) {

@@ -54,3 +54,29 @@ def test_queued_force_destinations():
     assert np.array_equal(pageable, want)
     assert np.array_equal(odd.numpy()[4:28].copy().view(np.float64), want)
     g.close()
+
+
+def test_queued_force_at_the_end_of_its_range():
+    """The last three doubles of a registered range and of a device allocation."""
+    import torch
+
+    g, case = sphere(32, 9.0)
+    want = getSphereForce(g, case)
+    page = 4096
+    raw = np.zeros(3 * page, dtype=np.uint8)
+    start = -raw.ctypes.data % page  # one page of it registered, pageable memory behind
+    host = raw[start:start + page]
+    cudart = torch.cuda.cudart()
+    assert int(cudart.cudaHostRegister(host.ctypes.data, page, 0)) == 0
+    try:
+        device = torch.zeros(1 << 20, dtype=torch.float64, device="cuda")
+        getSphereForceAsync(g, case, host.ctypes.data + page - 24)
+        getSphereForceAsync(g, case, device.data_ptr() + 8 * ((1 << 20) - 3))
+        g.synchronize()
+        torch.cuda.synchronize()
+        assert np.array_equal(host[-24:].copy().view(np.float64), want)
+        assert np.array_equal(device[-3:].cpu().numpy(), want)
+        assert not host[:-24].any() and not raw[start + page:].any()
+    finally:
+        assert int(cudart.cudaHostUnregister(host.ctypes.data)) == 0
+    g.close()
