@@ -46,7 +46,7 @@ __attribute__((visibility("hidden"))) void psl_detail_set_last_error(const std::
     if (!(cond)) return fail(code, msg); \
   } while (0)
 
-static constexpr int kForceBlocks = 512;  // below 2^16 (force_kernel's block count)
+static constexpr int kForceBlocks = 512;
 
 template <typename S>
 static GridView<S> view(const psl_grid* g) {
@@ -885,13 +885,12 @@ static int enqueue_sphere_force(psl_grid* g, const psl_sphere_case* sc, double* 
   if (i1 <= i0 || j1 <= j0 || k1 <= k0) return 1;
   const int si = i1 - i0, sj = j1 - j0, sk = k1 - k0;
   const int nb = (int)std::min<long long>(kForceBlocks, ((long long)si * sj * sk + kForceThreads - 1) / kForceThreads);
-  g->force_calls = g->force_calls % 0xffffu + 1;  // 1 .. 65535
   unsigned int* done = reinterpret_cast<unsigned int*>(g->scratch + kForceBlocks * 3 + 3);
   PSL_CUDA(with_storage(g->storage, [&](auto s) {
     using S = decltype(s);
     return launch_dependent(!stream_capturing(g->stream), force_kernel<S>, dim3(nb), kForceThreads, 0, g->stream, view<S>(g),
                             g->marker, I.cell_count_x, I.cell_count_y, i0, j0, k0, si, sj, sk, g->scratch, done,
-                            g->force_calls, out);
+                            out);
   }));
   return PSL_OK;
 }

@@ -48,7 +48,6 @@ struct psl_grid {
   cudaStream_t stream = 0;
   unsigned int* health = nullptr;   // [0] health bits
   double* scratch = nullptr;        // force partials (kForceBlocks x 3) + result (3) + block count (1)
-  unsigned int force_calls = 0;     // force reductions launched (force_kernel's call number)
   int device = 0;
   int batched = 0;                  // member of this many live batches (psl_batch.cu)
   float3 body = make_float3(0.f, 0.f, 0.f);  // uniform body force (customised update)

@@ -1094,16 +1094,13 @@ __global__ void __launch_bounds__(kForceThreads) force_partial_kernel(GridView<S
 
 // The force in one launch: the block that finishes last adds the partial sums in block order
 // (the sums and bits of force_partial_kernel followed by force_final_kernel) and writes the
-// three components to `out`, device memory or mapped host memory, so no copy follows.  A step
-// of the 128x64x64 sphere with its drag read every step took 42.9 us with two kernels and a
-// 24-byte copy behind the update; 33.1 us with this
-// kernel, both as dependent launches (37.2 us without).
-// `done`: blocks finished in the low 16 bits, the call's number above them: a count left by
-// another call starts anew, and the last block clears it (a replayed capture repeats its number).
+// three components to `out`, device memory or mapped host memory, so no copy follows.
+// `done` counts the finished blocks and wraps to zero by itself with the last one, so a replayed
+// capture finds it as a direct call does.
 template <typename S>
 __global__ void __launch_bounds__(kForceThreads)
     force_kernel(const __grid_constant__ GridView<S> g, const uint8_t* marker, int nx, int ny, int i0, int j0, int k0, int si,
-                 int sj, int sk, double* partial, unsigned int* done, unsigned int call, double* out) {
+                 int sj, int sk, double* partial, unsigned int* done, double* out) {
   constexpr int kChunk = 256;  // blocks per staged chunk
   __shared__ double stage[kChunk * 3];
   __shared__ bool last;
@@ -1112,18 +1109,8 @@ __global__ void __launch_bounds__(kForceThreads)
   force_partial(g, marker, nx, ny, i0, j0, k0, si, sj, sk, partial);
   if (threadIdx.x == 0) {
     __threadfence();  // the partial sums before the count
-    unsigned int seen = *(volatile unsigned int*)done, next;
-    for (;;) {
-      next = (seen >> 16) == call ? seen + 1 : (call << 16) + 1;
-      const unsigned int old = atomicCAS(done, seen, next);
-      if (old == seen) break;
-      seen = old;
-    }
-    last = (next & 0xffffu) == gridDim.x;
-    if (last) {
-      *done = 0;
-      __threadfence();
-    }
+    last = atomicInc(done, gridDim.x - 1) == gridDim.x - 1;
+    __threadfence();
   }
   __syncthreads();
   if (!last) return;

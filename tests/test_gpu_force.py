@@ -80,3 +80,39 @@ def test_queued_force_at_the_end_of_its_range():
     finally:
         assert int(cudart.cudaHostUnregister(host.ctypes.data)) == 0
     g.close()
+
+
+def test_replayed_captures_and_direct_calls_interleaved():
+    """Captured force calls over two boxes (a few blocks, and all 512 of the scratch) replayed with
+    direct calls in between: every result is the direct call's, bit for bit."""
+    import copy
+
+    import torch
+
+    g, small = sphere(64, 5.0)
+    large = copy.copy(small)
+    large.radius = 27.0  # the same solid cells inside a box of 55^3 cells
+    want = {"small": getSphereForce(g, small), "large": getSphereForce(g, large)}
+    got = {k: torch.zeros(3, dtype=torch.float64, pin_memory=True) for k in ("small", "large", "direct")}
+    stream = torch.cuda.Stream()
+    g.synchronize()
+    g.set_stream(stream.cuda_stream)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        getSphereForceAsync(g, small, got["small"].data_ptr())
+        getSphereForceAsync(g, large, got["large"].data_ptr())
+        getSphereForceAsync(g, small, got["small"].data_ptr())
+    for round_ in range(4):
+        for k in got:
+            got[k].fill_(float("nan"))
+        with torch.cuda.stream(stream):
+            graph.replay()
+            getSphereForceAsync(g, large if round_ % 2 else small, got["direct"].data_ptr())
+            graph.replay()
+        stream.synchronize()
+        for k in ("small", "large"):
+            assert np.array_equal(got[k].numpy(), want[k]), (round_, k)
+        assert np.array_equal(got["direct"].numpy(), want["large" if round_ % 2 else "small"]), round_
+    del graph
+    g.set_stream(0)
+    g.close()
