@@ -117,13 +117,13 @@ __device__ __forceinline__ void chimera_bwd(T& m0, T& m1, T& m2, const BwdCoef<T
   m2 = fp;
 }
 
-template <typename T>
+template <typename T, bool kPair = kPaired<T>>
 __device__ __forceinline__ void line_sums(const T (&f)[27], T (&sum)[3][3], T (&diff)[3][3], T (&pm)[3][3]) {
 #pragma unroll
   for (int i = 0; i < 3; ++i)
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
-      if constexpr (kPaired<T>) {
+      if constexpr (kPair) {
         if (i == 2) continue;  // with i = 0
         if (i == 0) {
           const FPair a(f[slot(0, j, 0)], f[slot(2, j, 0)]), b(f[slot(0, j, 1)], f[slot(2, j, 1)]),
@@ -147,7 +147,7 @@ __device__ __forceinline__ void line_sums(const T (&f)[27], T (&sum)[3][3], T (&
 
 // Central moments about (ux, uy, uz) from the z-line sums: K[i][j][k] = moment of order i
 // in x, j in y, k in z.
-template <typename T>
+template <typename T, bool kPair = kPaired<T>>
 __device__ __forceinline__ void transform_about(const T (&sum)[3][3], const T (&diff)[3][3], const T (&pm)[3][3], T ux,
                                                 T uy, T uz, T (&K)[3][3][3]) {
   const T uz2 = uz * uz, uy2 = uy * uy, ux2 = ux * ux;
@@ -155,7 +155,7 @@ __device__ __forceinline__ void transform_about(const T (&sum)[3][3], const T (&
   for (int i = 0; i < 3; ++i)
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
-      if constexpr (kPaired<T>) {
+      if constexpr (kPair) {
         if (i == 2) continue;  // with i = 0
         if (i == 0) {
           const FPair s(sum[0][j], sum[2][j]), d(diff[0][j], diff[2][j]), p(pm[0][j], pm[2][j]);
@@ -177,7 +177,7 @@ __device__ __forceinline__ void transform_about(const T (&sum)[3][3], const T (&
   for (int i = 0; i < 3; ++i)
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-      if constexpr (kPaired<T>) {
+      if constexpr (kPair) {
         if (i == 2) continue;
         if (i == 0) {
           FPair a(K[0][0][k], K[2][0][k]), b(K[0][1][k], K[2][1][k]), c(K[0][2][k], K[2][2][k]);
@@ -203,11 +203,11 @@ __device__ __forceinline__ void transform_about(const T (&sum)[3][3], const T (&
 
 // Forward transform of all 27 populations, returning rho, u and 1/rho; rho and the
 // momentum come from the z-line sums and differences of the first pass.
-template <typename T>
+template <typename T, bool kPair = kPaired<T>>
 __device__ __forceinline__ void central_moments(const T (&f)[27], T (&K)[3][3][3], T& rho, T& ux, T& uy, T& uz,
                                                 T& inv_rho) {
   T sum[3][3], diff[3][3], pm[3][3];
-  line_sums(f, sum, diff, pm);
+  line_sums<T, kPair>(f, sum, diff, pm);
   T sx[3], sy[3];
 #pragma unroll
   for (int i = 0; i < 3; ++i) sx[i] = (sum[i][0] + sum[i][2]) + sum[i][1];
@@ -222,14 +222,14 @@ __device__ __forceinline__ void central_moments(const T (&f)[27], T (&K)[3][3][3
   ux = jx * inv_rho;
   uy = jy * inv_rho;
   uz = jz * inv_rho;
-  transform_about(sum, diff, pm, ux, uy, uz, K);
+  transform_about<T, kPair>(sum, diff, pm, ux, uy, uz, K);
 }
 
 // Post-collision central moments (zero entries implicit) -> populations.
 // Inputs: k000 (= rho), first-order moments (already negated), relaxed second-order
 // cumulants s***, and inv_rho.  Higher central moments follow from the zero higher
 // cumulants (Geier 2015 eqs 81, 82, 84; include/applyCollision.h:178-200).
-template <typename T>
+template <typename T, bool kPair = kPaired<T>>
 __device__ __forceinline__ void populations_from_cumulants(T (&f)[27], T k000, T k100, T k010, T k001, T s200, T s020,
                                                            T s002, T s011, T s101, T s110, T inv_rho, T ux, T uy, T uz) {
   const T k211 = (s200 * s011 + T(2) * s101 * s110) * inv_rho;
@@ -266,7 +266,7 @@ __device__ __forceinline__ void populations_from_cumulants(T (&f)[27], T k000, T
   chimera_bwd<false, true, false>(G[0][2][1], G[1][2][1], G[2][2][1], bx);
   G[0][2][2] = k022; G[1][2][2] = T(0); G[2][2][2] = k222;
   chimera_bwd<true, false, true>(G[0][2][2], G[1][2][2], G[2][2][2], bx);
-  if constexpr (kPaired<T>) {
+  if constexpr (kPair) {
     // y and z passes with x slots 0 and 2 in pairs; of x slot 1, y slots 0 and 2 in the z pass
     const BwdCoef<FPair> by2(by), bz2(bz);
     FPair P[3][3];
@@ -407,11 +407,15 @@ __device__ __forceinline__ T collide(T (&f)[27], const RelaxationT<scalar_t<T>>&
 }
 
 // Moment rescaling across a 2:1 level change (include/gridRefinementFunctions.h:6-281).
+// In scalar operations: the transfer is bound by the latency of its gathers, and the pairs, which
+// need populations of two x slots at once, made the compiler order those loads worse (the same
+// bits; prolongation of the 512x256x256 sphere's block 96 -> 118 us in FP32, 91 -> 105 us in
+// FP16, of the 200x96x90 one 15 -> 20 us).
 template <typename T>
 __device__ __forceinline__ void rescale(T (&f)[27], bool coarse_to_fine) {
   T K[3][3][3];
   T rho, ux, uy, uz, inv_rho;
-  central_moments(f, K, rho, ux, uy, uz, inv_rho);
+  central_moments<T, false>(f, K, rho, ux, uy, uz, inv_rho);
   const T p200 = K[2][0][0], p020 = K[0][2][0], p002 = K[0][0][2];
   const T p011 = K[0][1][1], p101 = K[1][0][1], p110 = K[1][1][0];
   T c200, c020, c002, c011, c101, c110;
@@ -431,8 +435,8 @@ __device__ __forceinline__ void rescale(T (&f)[27], bool coarse_to_fine) {
     c110 = T(2) * p110;
   }
   // rescaleF negates the first-order central moments too (gridRefinementFunctions.h:154-156)
-  populations_from_cumulants(f, K[0][0][0], -K[1][0][0], -K[0][1][0], -K[0][0][1], c200, c020, c002, c011, c101, c110,
-                             inv_rho, ux, uy, uz);
+  populations_from_cumulants<T, false>(f, K[0][0][0], -K[1][0][0], -K[0][1][0], -K[0][0][1], c200, c020, c002, c011,
+                                       c101, c110, inv_rho, ux, uy, uz);
 }
 
 }  // namespace psl
