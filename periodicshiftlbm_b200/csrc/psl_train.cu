@@ -41,7 +41,12 @@ constexpr int kW1 = 0, kB1 = 320, kW2 = 352, kB2 = 1376, kW3 = 1408, kB3 = 1440,
 constexpr int kShift = 1441, kScale = 1451, kOutScale = 1461, kParams = 1462;
 constexpr int kMaxGradWarps = 14;
 constexpr int kGradBlocks = 148;  // one block per SM (159 KB of shared memory at 14 warps)
+// Tiles a warp adds up in FP32 before FP64 takes over: 128 samples a chain.  Larger batches run
+// in pieces of kPieceSamples, whose sums are added in FP64.  One chain over all of a batch of 2^22
+// equal samples (2,048 products each) was off by 2.9e-5 of the gradient.
+constexpr int kMaxTilesPerWarp = 4;
 constexpr int kTile = 32;         // samples per warp tile
+constexpr long long kPieceSamples = (long long)kGradBlocks * kMaxGradWarps * kMaxTilesPerWarp * kTile;
 constexpr int kLd = 36;           // floats per row of 32 samples: consecutive rows 4 banks apart
 
 int fail(int code, const std::string& msg) {
@@ -140,22 +145,22 @@ __device__ __forceinline__ float sum_scatter(const float (&v)[8], int sg) {
   return (up ? b[1] : b[0]) + __shfl_xor_sync(0xffffffffu, up ? b[0] : b[1], 1);
 }
 
-// Partial gradients of the batch samples [0, count): sample i is row first + i, or a
+// Partial gradients of the samples [lo, hi) of a batch of `count`: sample i is row first + i, or a
 // hashed row of [0, n) when `random`.  partial[block][0..kTrainable) gets the block's
-// gradient sums, partial[block][kTrainable] its loss sum.  Tile t of 32 samples belongs to
-// block t % gridDim.x, warp t / gridDim.x (cyclically).
+// gradient sums, partial[block][kTrainable] its loss sum.  Tile t of 32 samples (from lo, a
+// multiple of 32) belongs to block t % gridDim.x, warp t / gridDim.x (cyclically).
 //
 // What bounds it: instruction issue and latency, beside the two launches of a step (0.45
 // instructions per cycle and scheduler at 3.5 warps each).  Each lane holds a 4 x 8 tile of
 // the three passes (32 FMAs, two per instruction, from three 16-byte loads) and 8 x 4 of the
-// 32 x 32 weight gradient (128 FMAs from twelve); weight-gradient accumulators stay in
-// registers over all of a warp's tiles.  One training step of 65,536 samples: 60.3 us with one
+// 32 x 32 weight gradient (128 FMAs from twelve); the weight-gradient accumulators are kept
+// over all of a warp's tiles, one FP32 chain each, of at most kMaxTilesPerWarp tiles.  One training step of 65,536 samples: 60.3 us with one
 // thread per sample (every weight a broadcast load of its own, the weight gradients at two
 // loads per FMA) and three launches; 25.5 us now.  With scalar FMAs 27.7 us; with 64-sample
 // tiles (8 x 8 per lane, 7 warps per SM) 27.4 us without leaving room for the reduction's blocks.
 __global__ void __launch_bounds__(32 * kMaxGradWarps, 1)
     grad_kernel(const float* params, const float* __restrict__ X, const float* __restrict__ T, long long n, long long first,
-                long long count, int random, uint32_t seed, float* partial) {
+                long long lo, long long hi, long long count, int random, uint32_t seed, float* partial) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   GradWeights& W = *reinterpret_cast<GradWeights*>(smem_raw);
   GradTile* tiles = reinterpret_cast<GradTile*>(smem_raw + sizeof(GradWeights));
@@ -171,7 +176,7 @@ __global__ void __launch_bounds__(32 * kMaxGradWarps, 1)
   bool valid = false;
   auto gather = [&](long long tile) {
     const long long i = tile * kTile + c0;
-    valid = i < count;
+    valid = i < hi;
     long long row = 0;
     if (valid) {
       row = first + i;
@@ -184,8 +189,8 @@ __global__ void __launch_bounds__(32 * kMaxGradWarps, 1)
     for (int k = 0; k < kMlpIn / 2; ++k) raw[k] = reinterpret_cast<const float2*>(X + row * kMlpIn)[k];
     target = T[row];
   };
-  long long tile = blockIdx.x + (long long)gridDim.x * warp;
-  if (tile * kTile < count) gather(tile);
+  long long tile = lo / kTile + blockIdx.x + (long long)gridDim.x * warp;
+  if (tile * kTile < hi) gather(tile);
 
   grid_wait();
   grid_release();
@@ -227,7 +232,7 @@ __global__ void __launch_bounds__(32 * kMaxGradWarps, 1)
     for (int i = 0; i < 5; ++i) g1[m][i] = 0.f;
   }
 
-  for (; tile * kTile < count; tile += (long long)gridDim.x * warps) {
+  for (; tile * kTile < hi; tile += (long long)gridDim.x * warps) {
     const bool ok = valid;
     const float t = target / W.out_scale;
 #pragma unroll
@@ -332,7 +337,7 @@ __global__ void __launch_bounds__(32 * kMaxGradWarps, 1)
     __syncwarp();
     // the next tile's samples arrive during the last product
     const long long next = tile + (long long)gridDim.x * warps;
-    if (next * kTile < count) gather(next);
+    if (next * kTile < hi) gather(next);
     // ---- weight gradient of layer 1: d1 (32 x samples) times x^T ----
 #pragma unroll 1
     for (int c = kTile / 2 * half; c < kTile / 2 * (half + 1); c += 4) {
@@ -384,8 +389,9 @@ __global__ void __launch_bounds__(32 * kMaxGradWarps, 1)
   }
 }
 
-// grad[e] = sum over blocks of partial[block][e] in FP64, grad[kTrainable] the mean loss; with
-// kAdam also the Adam update of the parameter.  Eight entries (one 32-byte sector of a block's
+// grad[e] = sum over blocks of partial[block][e] in FP64, added to grad[e] unless this is the
+// batch's first piece; with its last, grad[kTrainable] becomes the mean loss and, with kAdam, the
+// parameter takes its Adam update.  Eight entries (one 32-byte sector of a block's
 // row) per block and 16 groups of threads that take every 16th row each, then the 16 sums in
 // order.  One thread per entry summing all rows kept six blocks busy with a serial chain of
 // loads (16.3 us at 296 rows, Adam a launch of its own at 4.2 us).  128 threads of at most 32
@@ -401,7 +407,8 @@ struct AdamParams {
 constexpr int kReduceEntries = 8, kReduceGroups = 16;
 template <bool kAdam>
 __global__ void __launch_bounds__(kReduceEntries * kReduceGroups, 16)
-    reduce_kernel(const float* partial, int blocks, long long count, double* grad, AdamParams ad) {
+    reduce_kernel(const float* partial, int blocks, long long count, bool first_piece, bool last_piece, double* grad,
+                  AdamParams ad) {
   __shared__ double part[kReduceGroups][kReduceEntries];
   const int entry = threadIdx.x % kReduceEntries, group = threadIdx.x / kReduceEntries;
   const int e = blockIdx.x * kReduceEntries + entry;
@@ -423,8 +430,9 @@ __global__ void __launch_bounds__(kReduceEntries * kReduceGroups, 16)
   s = 0.0;
 #pragma unroll
   for (int w = 0; w < kReduceGroups; ++w) s += part[w][entry];
-  grad[e] = e == kTrainable ? s / (double)count : s;
-  if (!kAdam || e >= kTrainable) return;
+  if (!first_piece) s += grad[e];
+  grad[e] = last_piece && e == kTrainable ? s / (double)count : s;
+  if (!kAdam || !last_piece || e >= kTrainable) return;
   const float g = (float)s;
   const float mm = ad.beta1 * ad.m[e] + (1.f - ad.beta1) * g;
   const float vv = ad.beta2 * ad.v[e] + (1.f - ad.beta2) * g * g;
@@ -573,20 +581,22 @@ struct psl_sgs_trainer {
 namespace {
 
 // One warp per 32-sample tile while that many warps fit (14 per SM), so that a batch of 65,536
-// samples is one tile per warp on 148 x 14 warps and a small batch spreads over the SMs.
+// samples is one tile per warp on 148 x 14 warps and a small batch spreads over the SMs; a batch of
+// more than kPieceSamples in pieces of that size.
 int run_gradient(psl_sgs_trainer* t, long long first, long long count, int random, uint32_t seed, const AdamParams* adam) {
-  const long long tiles = (count + kTile - 1) / kTile;
-  const int blocks = (int)std::min<long long>(kGradBlocks, tiles);
-  const int warps = (int)std::min<long long>(kMaxGradWarps, (tiles + blocks - 1) / blocks);
-  TRAIN_CUDA(launch_dependent(true, grad_kernel, dim3(blocks), 32 * warps, grad_smem(warps), t->stream, (const float*)t->params,
-                              (const float*)t->X, (const float*)t->T, t->count, first, count, random, seed, t->partial));
   const unsigned int nb = (kTrainable + kReduceEntries) / kReduceEntries, threads = kReduceEntries * kReduceGroups;
-  if (adam)
-    TRAIN_CUDA(launch_dependent(true, reduce_kernel<true>, dim3(nb), threads, 0, t->stream, (const float*)t->partial, blocks,
-                                count, t->grad, *adam));
-  else
-    TRAIN_CUDA(launch_dependent(true, reduce_kernel<false>, dim3(nb), threads, 0, t->stream, (const float*)t->partial, blocks,
-                                count, t->grad, AdamParams{}));
+  for (long long lo = 0; lo < count; lo += kPieceSamples) {
+    const long long hi = std::min(count, lo + kPieceSamples);
+    const long long tiles = (hi - lo + kTile - 1) / kTile;
+    const int blocks = (int)std::min<long long>(kGradBlocks, tiles);
+    const int warps = (int)std::min<long long>(kMaxGradWarps, (tiles + blocks - 1) / blocks);
+    TRAIN_CUDA(launch_dependent(true, grad_kernel, dim3(blocks), 32 * warps, grad_smem(warps), t->stream,
+                                (const float*)t->params, (const float*)t->X, (const float*)t->T, t->count, first, lo, hi, count,
+                                random, seed, t->partial));
+    TRAIN_CUDA(launch_dependent(true, adam ? reduce_kernel<true> : reduce_kernel<false>, dim3(nb), threads, 0, t->stream,
+                                (const float*)t->partial, blocks, count, lo == 0, hi == count, t->grad,
+                                adam ? *adam : AdamParams{}));
+  }
   return PSL_OK;
 }
 
