@@ -244,36 +244,96 @@ PSL_HDI void bwd_full_w(T& a, T& b, T& c, const BwdAxis<T>& k, float wpm, float 
   c = h + e;
 }
 
-#if defined(__CUDA_ARCH__)
 // Two triples at once in packed FP32 (sm_100: one instruction, each half rounded as the scalar
-// operation): the triples at x = -1 and x = +1 share their coefficients and weights.  The
-// 16-bit updates are bound by instruction issue beside 64-byte row accesses; the pairs leave out
-// about 46 instructions per cell, registers unchanged: 251x117x125 BF16 grid 130.0 -> 127.2 us
-// per step, refined 256x128x128 FP16 sphere 232.4 -> 227.5 us, 129x129x128 FP16 box with the
-// closure 105 -> 98.4 us.
-struct BwdAxis2 {
-  float2 hu2, hu, tu;
-  __device__ __forceinline__ explicit BwdAxis2(const BwdAxis<float>& k)
-      : hu2(make_float2(k.hu2, k.hu2)), hu(make_float2(k.hu, k.hu)), tu(make_float2(k.tu, k.tu)) {}
+// operation; host builds take the halves one by one): the triples at x = -1 and x = +1 share
+// their coefficients and weights.  The 16-bit updates are bound by instruction issue beside
+// 64-byte row accesses; the pairs leave out about 46 instructions per cell, registers unchanged:
+// 251x117x125 BF16 grid 130.0 -> 127.2 us per step, refined 256x128x128 FP16 sphere
+// 232.4 -> 227.5 us, 129x129x128 FP16 box with the closure 105 -> 98.4 us.
+#if defined(__CUDACC__)
+using GPair = float2;
+#else
+struct GPair {
+  float x, y;
 };
-__device__ __forceinline__ float2 both(float a) { return make_float2(a, a); }
-__device__ __forceinline__ void bwd_full2(float2& a, float2& b, float2& c, const BwdAxis2& k) {
-  const float2 m0 = a, m1 = b, m2 = c;
-  const float2 h = __ffma2_rn(k.hu2, m0, __ffma2_rn(k.tu, m1, m2));
-  const float2 e = __ffma2_rn(k.hu, m0, m1);
-  a = __ffma2_rn(both(-1.f), e, h);
-  b = __ffma2_rn(both(-2.f), h, m0);
-  c = __fadd2_rn(h, e);
-}
-__device__ __forceinline__ void bwd_full_w2(float2& a, float2& b, float2& c, const BwdAxis2& k, float wpm, float w0) {
-  const float2 m0 = a, m1 = b, m2 = c;
-  const float2 h = __fadd2_rn(__ffma2_rn(k.hu2, m0, __ffma2_rn(k.tu, m1, m2)), both(-wpm));
-  const float2 e = __ffma2_rn(k.hu, m0, m1);
-  a = __ffma2_rn(both(-1.f), e, h);
-  b = __ffma2_rn(both(-2.f), h, __fadd2_rn(m0, both(-(w0 + 2.f * wpm))));
-  c = __fadd2_rn(h, e);
-}
 #endif
+PSL_HDI GPair gpair(float a, float b) {
+  GPair p;
+  p.x = a;
+  p.y = b;
+  return p;
+}
+PSL_HDI GPair both(float a) { return gpair(a, a); }
+PSL_HDI GPair pair_fma(GPair a, GPair b, GPair c) {
+#if defined(__CUDA_ARCH__)
+  return __ffma2_rn(a, b, c);
+#else
+  return gpair(gfma(a.x, b.x, c.x), gfma(a.y, b.y, c.y));
+#endif
+}
+PSL_HDI GPair pair_add(GPair a, GPair b) {
+#if defined(__CUDA_ARCH__)
+  return __fadd2_rn(a, b);
+#else
+  return gpair(a.x + b.x, a.y + b.y);
+#endif
+}
+struct BwdAxis2 {
+  GPair hu2, hu, tu;
+  PSL_HDI explicit BwdAxis2(const BwdAxis<float>& k) : hu2(both(k.hu2)), hu(both(k.hu)), tu(both(k.tu)) {}
+};
+PSL_HDI void bwd_full2(GPair& a, GPair& b, GPair& c, const BwdAxis2& k) {
+  const GPair m0 = a, m1 = b, m2 = c;
+  const GPair h = pair_fma(k.hu2, m0, pair_fma(k.tu, m1, m2));
+  const GPair e = pair_fma(k.hu, m0, m1);
+  a = pair_fma(both(-1.f), e, h);
+  b = pair_fma(both(-2.f), h, m0);
+  c = pair_add(h, e);
+}
+PSL_HDI void bwd_full_w2(GPair& a, GPair& b, GPair& c, const BwdAxis2& k, float wpm, float w0) {
+  const GPair m0 = a, m1 = b, m2 = c;
+  const GPair h = pair_add(pair_fma(k.hu2, m0, pair_fma(k.tu, m1, m2)), both(-wpm));
+  const GPair e = pair_fma(k.hu, m0, m1);
+  a = pair_fma(both(-1.f), e, h);
+  b = pair_fma(both(-2.f), h, pair_add(m0, both(-(w0 + 2.f * wpm))));
+  c = pair_add(h, e);
+}
+
+// The y and z passes: G[x-slot][y-order][z-order] after the x pass -> g.  y: x slots 0 and 2 in
+// pairs, x slot 1 alone; z, weights subtracted: the same pairs, and y slots 0 and 2 of x slot 1.
+PSL_HDI void backward_yz_g(float (&G)[3][3][3], const BwdAxis<float>& by, const BwdAxis<float>& bz, float (&g)[27]) {
+  GPair P[3][3];
+#pragma unroll
+  for (int b = 0; b < 3; ++b)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) P[b][c] = gpair(G[0][b][c], G[2][b][c]);
+  const BwdAxis2 by2(by), bz2(bz);
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    bwd_full2(P[0][c], P[1][c], P[2][c], by2);
+    bwd_full(G[1][0][c], G[1][1][c], G[1][2][c], by);
+  }
+#pragma unroll
+  for (int b = 0; b < 3; ++b) {
+    bwd_full_w2(P[b][0], P[b][1], P[b][2], bz2, lattice_weight(slot(0, b, 0)), lattice_weight(slot(0, b, 1)));
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      g[slot(0, b, c)] = P[b][c].x;
+      g[slot(2, b, c)] = P[b][c].y;
+    }
+  }
+  GPair m0 = gpair(G[1][0][0], G[1][2][0]), m1 = gpair(G[1][0][1], G[1][2][1]), m2 = gpair(G[1][0][2], G[1][2][2]);
+  bwd_full_w2(m0, m1, m2, bz2, lattice_weight(slot(1, 0, 0)), lattice_weight(slot(1, 0, 1)));
+  bwd_full_w(G[1][1][0], G[1][1][1], G[1][1][2], bz, lattice_weight(slot(1, 1, 0)), lattice_weight(slot(1, 1, 1)));
+  g[slot(1, 0, 0)] = m0.x;
+  g[slot(1, 2, 0)] = m0.y;
+  g[slot(1, 0, 1)] = m1.x;
+  g[slot(1, 2, 1)] = m1.y;
+  g[slot(1, 0, 2)] = m2.x;
+  g[slot(1, 2, 2)] = m2.y;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) g[slot(1, 1, c)] = G[1][1][c];
+}
 
 // Post-collision g' = f' - w from rho, u and the relaxed second-order central moments
 // s** (first-order central moments zero, third-order cumulants zero; the fourth- and
@@ -319,59 +379,7 @@ PSL_HDI void populations_g(T (&g)[27], T rho, T inv_rho, T ux, T uy, T uz, T s20
   bwd_odd(G[0][2][1], G[1][2][1], G[2][2][1], xm, x0, xp);
   G[0][2][2] = k022; G[1][2][2] = zero; G[2][2][2] = k222;
   bwd_even(G[0][2][2], G[1][2][2], G[2][2][2], bx);
-#if defined(__CUDA_ARCH__)
-  // y pass: x slots 0 and 2 in pairs, x slot 1 alone
-  float2 P[3][3];
-#pragma unroll
-  for (int b = 0; b < 3; ++b)
-#pragma unroll
-    for (int c = 0; c < 3; ++c) P[b][c] = make_float2(G[0][b][c], G[2][b][c]);
-  const BwdAxis2 by2(by), bz2(bz);
-#pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    bwd_full2(P[0][c], P[1][c], P[2][c], by2);
-    bwd_full(G[1][0][c], G[1][1][c], G[1][2][c], by);
-  }
-  // z pass, weights subtracted: the same pairs, and y slots 0 and 2 of x slot 1
-#pragma unroll
-  for (int b = 0; b < 3; ++b) {
-    bwd_full_w2(P[b][0], P[b][1], P[b][2], bz2, lattice_weight(slot(0, b, 0)), lattice_weight(slot(0, b, 1)));
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      g[slot(0, b, c)] = P[b][c].x;
-      g[slot(2, b, c)] = P[b][c].y;
-    }
-  }
-  float2 m0 = make_float2(G[1][0][0], G[1][2][0]), m1 = make_float2(G[1][0][1], G[1][2][1]),
-         m2 = make_float2(G[1][0][2], G[1][2][2]);
-  bwd_full_w2(m0, m1, m2, bz2, lattice_weight(slot(1, 0, 0)), lattice_weight(slot(1, 0, 1)));
-  bwd_full_w(G[1][1][0], G[1][1][1], G[1][1][2], bz, lattice_weight(slot(1, 1, 0)), lattice_weight(slot(1, 1, 1)));
-  g[slot(1, 0, 0)] = m0.x;
-  g[slot(1, 2, 0)] = m0.y;
-  g[slot(1, 0, 1)] = m1.x;
-  g[slot(1, 2, 1)] = m1.y;
-  g[slot(1, 0, 2)] = m2.x;
-  g[slot(1, 2, 2)] = m2.y;
-#pragma unroll
-  for (int c = 0; c < 3; ++c) g[slot(1, 1, c)] = G[1][1][c];
-#else
-  // y pass
-#pragma unroll
-  for (int a = 0; a < 3; ++a)
-#pragma unroll
-    for (int c = 0; c < 3; ++c) bwd_full(G[a][0][c], G[a][1][c], G[a][2][c], by);
-  // z pass, weights subtracted
-#pragma unroll
-  for (int a = 0; a < 3; ++a)
-#pragma unroll
-    for (int b = 0; b < 3; ++b) {
-      T m0 = G[a][b][0], m1 = G[a][b][1], m2 = G[a][b][2];
-      bwd_full_w(m0, m1, m2, bz, lattice_weight(slot(a, b, 0)), lattice_weight(slot(a, b, 1)));
-      g[slot(a, b, 0)] = m0;
-      g[slot(a, b, 1)] = m1;
-      g[slot(a, b, 2)] = m2;
-    }
-#endif
+  backward_yz_g(G, by, bz, g);
 }
 
 // Relaxation at shear rate w (bulk at 1; include/applyCollision.h:119-200) from D, then
