@@ -54,3 +54,31 @@ def test_scalar_update_of_every_cell_kind(dims, storage):
         # 16-bit flow: the collision uses the unrounded populations, f read back is rounded to 2^-11 of f - w
         assert np.max(np.abs(T1[:, c] - want)) < (2e-6 if storage == "f32" else 2e-3), (c, kind[c])
     g.close()
+
+
+@pytest.mark.parametrize("dims", [(5, 3, 2), (64, 64, 63), (64, 64, 64)])  # below, just below and at 1 MiB per row
+def test_scalar_populations_through_pinned_and_pageable_memory(dims):
+    import ctypes
+
+    import torch
+
+    from periodicshiftlbm_b200._lib import call
+
+    g = GridStruct(InfoStruct(cellCountX=dims[0], cellCountY=dims[1], cellCountZ=dims[2], nu=0.02))
+    n = g.cellCount
+    g.enableScalarTransport(0.7)
+    g.shifter = (np.arange(27) * 7919 % n).astype(np.int32)
+    want = np.random.default_rng(n).uniform(0.0, 1.0, (27, n)).astype(np.float32)
+    pinned = torch.from_numpy(want.copy()).pin_memory()
+    back = torch.zeros((27, n), dtype=torch.float32, pin_memory=True)
+    for write_pinned in (True, False):
+        g.TArray = np.zeros((27, n), np.float32)
+        if write_pinned:
+            call("psl_set_scalar_populations", g.handle, ctypes.c_void_p(pinned.data_ptr()))
+        else:
+            g.TArray = want
+        assert np.array_equal(g.TArray, want)
+        back.zero_()
+        call("psl_get_scalar_populations", g.handle, ctypes.c_void_p(back.data_ptr()))
+        assert np.array_equal(back.numpy(), want)
+    g.close()
