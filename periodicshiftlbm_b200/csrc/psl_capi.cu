@@ -614,8 +614,8 @@ int psl_apply_local_cell_update(psl_grid* g) {
         }
         sp.givenT = g->givenT;
         sp.tauT = g->tauT;
-        return launch_dependent(false, step_scalar_kernel<S>, dim3(blocks_for(g->n, kStepThreads)),
-                                kStepThreads, 0, g->stream, sp);
+        step_scalar_kernel<S><<<blocks_for(g->n, kStepThreads), kStepThreads, 0, g->stream>>>(sp);
+        return cudaGetLastError();
       }
       return cudaErrorInvalidValue;
     }));
@@ -644,8 +644,8 @@ int psl_apply_local_cell_update(psl_grid* g) {
         cp.base.rx = relaxation<float>(g);
         cp.base.health = g->health;
         cp.body = g->body;
-        return launch_dependent(false, step_custom_kernel<S>, dim3(blocks_for(g->n, kStepThreads)),
-                                kStepThreads, 0, g->stream, cp);
+        step_custom_kernel<S><<<blocks_for(g->n, kStepThreads), kStepThreads, 0, g->stream>>>(cp);
+        return cudaGetLastError();
       }
       return cudaErrorInvalidValue;
     }));

@@ -23,7 +23,7 @@ namespace psl {
 __device__ __forceinline__ float fmat(float a, float b, float c) { return fmaf(a, b, c); }
 __device__ __forceinline__ double fmat(double a, double b, double c) { return fma(a, b, c); }
 
-// Scalar type of an arithmetic type (the half of a packed pair).
+// Scalar type of an arithmetic type.
 template <typename T>
 struct scalar_of {
   using type = T;
@@ -44,10 +44,6 @@ struct FPair {
   __device__ __forceinline__ explicit FPair(float a) : v(make_float2(a, a)) {}
   __device__ __forceinline__ FPair(float a, float b) : v(make_float2(a, b)) {}
   __device__ __forceinline__ explicit FPair(float2 a) : v(a) {}
-};
-template <>
-struct scalar_of<FPair> {
-  using type = float;
 };
 __device__ __forceinline__ FPair operator+(FPair a, FPair b) { return FPair(__fadd2_rn(a.v, b.v)); }
 __device__ __forceinline__ FPair operator-(FPair a, FPair b) { return FPair(__ffma2_rn(make_float2(-1.f, -1.f), b.v, a.v)); }

@@ -304,8 +304,10 @@ __device__ __forceinline__ void local_cell_update(int kind, uint8_t m, T (&f)[27
 
 // Population addressing of the update kernels:
 //   kAddrView   64-bit row pointers with the periodic wrap (GridView)
-//   kAddrIndex  base + 32-bit row offsets with the wrap (RowIndex; 27 rows + N < 2^32 elements)
-//   kAddrFlat   base + 32-bit row offsets without the wrap, on rows mapped twice
+//   kAddrIndex  with the wrap, 27 rows + N < 2^32 elements: FP32 the cell's byte address + 64-bit
+//               byte offsets (FlatIndex, limits of RowIndex), else base + 32-bit row offsets (RowIndex)
+//   kAddrFlat   without the wrap, on rows mapped twice: the cell's byte address + 64-bit byte
+//               offsets (FlatIndex)
 enum RowAddr : int { kAddrView = 0, kAddrIndex = 1, kAddrFlat = 2 };
 
 template <typename A, int kAddr, typename S>
@@ -479,6 +481,8 @@ struct CustomParams {
 //                                  M35Full/m35Main.cu:101-119)
 //   every collided cell            plus the uniform body force, collided with the forcing
 //                                  collision (M40Impeller/applyCollisionCustomized.h:6-16)
+// Launched the ordinary way: with the waits of a dependent launch in the FP32 kernel a step of
+// 256x98x128 cells with its periodic copy took 129.1 us against 125.5 (64x24x32 cells 6.2 against 8.2).
 template <typename S>
 __global__ void __launch_bounds__(kStepThreads) step_custom_kernel(const __grid_constant__ CustomParams<S> cp) {
   const StepParams<S>& p = cp.base;

@@ -7,6 +7,10 @@
 // that of the kernel ahead), and grid_release after it, so that the blocks of the next kernel
 // start only once everything before this kernel is complete and visible.  Both are no-ops in a
 // kernel launched the ordinary way.
+//
+// One exception: the training samples, which grad_kernel reads before grid_wait (psl_train.cu).
+// Whoever writes them waits for the device before returning to the caller, so no kernel that a
+// grad_kernel can overlap writes them.
 #pragma once
 #include <cuda_runtime.h>
 

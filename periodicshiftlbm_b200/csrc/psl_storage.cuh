@@ -22,7 +22,8 @@ enum StorageKind : int { kStoreF32 = 0, kStoreF16 = 1, kStoreBF16 = 2, kStoreF64
 // 128 (FP32) contiguous bytes of a row, and the warps of the next cells read the rest of the
 // same lines.  FP32: ordinary loads, since a dependent launch's blocks start before the kernel
 // ahead has written these values and load them after grid_wait, out of which their index comes
-// (psl_launch.cuh).  16-bit: the read-only path, in kernels launched the ordinary way.
+// (psl_launch.cuh); the FP32 kernels launched the ordinary way (customised, scalar, learned, batch)
+// share them.  16-bit: the read-only path, in kernels launched the ordinary way only.
 __device__ __forceinline__ float ldg_row(const float* p) {
   float v;
   asm("ld.global.L2::256B.f32 %0, [%1];" : "=f"(v) : "l"(p));

@@ -150,8 +150,8 @@ __device__ __forceinline__ float sum_scatter(const float (&v)[8], int sg) {
 // gradient sums, partial[block][kTrainable] its loss sum.  Tile t of 32 samples (from lo, a
 // multiple of 32) belongs to block t % gridDim.x, warp t / gridDim.x (cyclically).
 //
-// What bounds it: instruction issue and latency, beside the two launches of a step (0.45
-// instructions per cycle and scheduler at 3.5 warps each).  Each lane holds a 4 x 8 tile of
+// What bounds it: instruction issue and latency at 3.5 warps per scheduler, beside the two launches
+// of a step.  Each lane holds a 4 x 8 tile of
 // the three passes (32 FMAs, two per instruction, from three 16-byte loads) and 8 x 4 of the
 // 32 x 32 weight gradient (128 FMAs from twelve); the weight-gradient accumulators are kept
 // over all of a warp's tiles, one FP32 chain each, of at most kMaxTilesPerWarp tiles.  One training step of 65,536 samples: 60.3 us with one
@@ -170,7 +170,8 @@ __global__ void __launch_bounds__(32 * kMaxGradWarps, 1)
   const int c0 = 4 * sg + og;  // this lane gathers sample c0 of a tile and evaluates its loss
 
   // the samples do not depend on the kernel ahead (which may still be updating the
-  // parameters): fetch the first tile's before waiting for it
+  // parameters): fetch the first tile's before waiting for it.  Safe, also through read-only
+  // loads, because both functions that add samples wait for the stream before they return.
   float2 raw[kMlpIn / 2] = {};
   float target = 0.f;
   bool valid = false;
@@ -664,7 +665,7 @@ int psl_sgs_trainer_add_samples(psl_sgs_trainer* t, const float* features, const
   TRAIN_CUDA(cudaMemcpyAsync(t->X + t->count * kMlpIn, features, (size_t)n * kMlpIn * sizeof(float),
                              cudaMemcpyHostToDevice, t->stream));
   TRAIN_CUDA(cudaMemcpyAsync(t->T + t->count, targets, (size_t)n * sizeof(float), cudaMemcpyHostToDevice, t->stream));
-  TRAIN_CUDA(cudaStreamSynchronize(t->stream));
+  TRAIN_CUDA(cudaStreamSynchronize(t->stream));  // required: grad_kernel reads samples before its grid_wait
   t->count += n;
   return PSL_OK;
 }
@@ -713,7 +714,7 @@ int psl_sgs_trainer_add_filtered(psl_sgs_trainer* t, psl_grid* fine, int M, int 
   }
   target_kernel<<<nb, 256, 0, t->stream>>>(rec, M, stride, (int)(phase % stride), t->X, t->T, t->count);
   cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess) e = cudaStreamSynchronize(t->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(t->stream);  // required: grad_kernel reads samples before its grid_wait
   cudaFree(rec);
   if (e != cudaSuccess) return fail(PSL_ERR_CUDA, std::string("psl_sgs_trainer_add_filtered: ") + cudaGetErrorString(e));
   t->count += selected;
