@@ -533,8 +533,13 @@ def run_reference(args):
     rank, world, _ = dist_env()
     if rank != 0:
         return
-    cfg = workload(args)
     lib, kind = _ref_lib()
+    if kind != "reference":  # a restatement of the reference is not the reference
+        print(json.dumps({"impl": "reference",
+                          "unavailable": "the reference's sources are not on this machine and oracle/_ref/libpsl_ref.so "
+                                         "was not built from them"}), flush=True)
+        return
+    cfg = workload(args)
     sim = lib.sim(_ref_case(cfg))
     budget_s = 150.0
     for _ in range(min(args.warmup, 1)):

@@ -57,3 +57,16 @@ def test_reference_arm_runs_on_rank_zero_only(monkeypatch, capsys):
     args = bench.parse()
     bench.run_reference(args)  # returns before any work on a rank other than 0
     assert capsys.readouterr().out == ""
+
+
+def test_reference_arm_without_the_reference_reports_no_number(monkeypatch, capsys):
+    """Where the reference's own code was not built, the arm says so instead of timing the oracle."""
+    import json
+
+    import oracle.bindings as bindings
+
+    monkeypatch.setattr(bindings, "ref_available", lambda: False)
+    monkeypatch.setattr(sys, "argv", ["bench.py", "--impl", "reference"])
+    bench.run_reference(bench.parse())
+    line = json.loads(capsys.readouterr().out)
+    assert line["impl"] == "reference" and line["unavailable"] and "value" not in line
