@@ -145,10 +145,10 @@ __device__ __forceinline__ float sum_scatter(const float (&v)[8], int sg) {
   return (up ? b[1] : b[0]) + __shfl_xor_sync(0xffffffffu, up ? b[0] : b[1], 1);
 }
 
-// Partial gradients of the samples [lo, hi) of a batch of `count`: sample i is row first + i, or a
-// hashed row of [0, n) when `random`.  partial[block][0..kTrainable) gets the block's
-// gradient sums, partial[block][kTrainable] its loss sum.  Tile t of 32 samples (from lo, a
-// multiple of 32) belongs to block t % gridDim.x, warp t / gridDim.x (cyclically).
+// Partial gradients of `count` samples of a batch of `total`: sample i is row first + i, or when
+// `random` the row of [0, n) that the hash of first + i gives.  partial[block][0..kTrainable) gets
+// the block's gradient sums, partial[block][kTrainable] its loss sum.  Tile t of 32
+// samples belongs to block t % gridDim.x, warp t / gridDim.x (cyclically).
 //
 // What bounds it: instruction issue and latency at 3.5 warps per scheduler, beside the two launches
 // of a step.  Each lane holds a 4 x 8 tile of
@@ -160,7 +160,7 @@ __device__ __forceinline__ float sum_scatter(const float (&v)[8], int sg) {
 // tiles (8 x 8 per lane, 7 warps per SM) 27.4 us without leaving room for the reduction's blocks.
 __global__ void __launch_bounds__(32 * kMaxGradWarps, 1)
     grad_kernel(const float* params, const float* __restrict__ X, const float* __restrict__ T, long long n, long long first,
-                long long lo, long long hi, long long count, int random, uint32_t seed, float* partial) {
+                long long count, long long total, int random, uint32_t seed, float* partial) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   GradWeights& W = *reinterpret_cast<GradWeights*>(smem_raw);
   GradTile* tiles = reinterpret_cast<GradTile*>(smem_raw + sizeof(GradWeights));
@@ -177,12 +177,12 @@ __global__ void __launch_bounds__(32 * kMaxGradWarps, 1)
   bool valid = false;
   auto gather = [&](long long tile) {
     const long long i = tile * kTile + c0;
-    valid = i < hi;
+    valid = i < count;
     long long row = 0;
     if (valid) {
       row = first + i;
       if (random) {
-        const uint32_t v = mix32(seed ^ mix32((uint32_t)i * 2654435761u + (uint32_t)(i >> 32)));
+        const uint32_t v = mix32(seed ^ mix32((uint32_t)row * 2654435761u + (uint32_t)(row >> 32)));
         row = n <= 0xffffffffll ? (long long)(v % (uint32_t)n) : (long long)v;
       }
     }
@@ -190,8 +190,8 @@ __global__ void __launch_bounds__(32 * kMaxGradWarps, 1)
     for (int k = 0; k < kMlpIn / 2; ++k) raw[k] = reinterpret_cast<const float2*>(X + row * kMlpIn)[k];
     target = T[row];
   };
-  long long tile = lo / kTile + blockIdx.x + (long long)gridDim.x * warp;
-  if (tile * kTile < hi) gather(tile);
+  long long tile = blockIdx.x + (long long)gridDim.x * warp;
+  if (tile * kTile < count) gather(tile);
 
   grid_wait();
   grid_release();
@@ -220,7 +220,7 @@ __global__ void __launch_bounds__(32 * kMaxGradWarps, 1)
   }
   __syncthreads();
 
-  const float inv_count = 1.f / (float)count;
+  const float inv_count = 1.f / (float)total;
   // gradient accumulators over the warp's tiles.  g2: rows o = og + 4 j, columns k = sg + 8 m;
   // g1: rows k = sg + 8 m, inputs 5 ig + i, half of the samples; b1, b2, w3: entry 8 og + sg
   const int ig = og & 1, half = og >> 1;
@@ -233,7 +233,7 @@ __global__ void __launch_bounds__(32 * kMaxGradWarps, 1)
     for (int i = 0; i < 5; ++i) g1[m][i] = 0.f;
   }
 
-  for (; tile * kTile < hi; tile += (long long)gridDim.x * warps) {
+  for (; tile * kTile < count; tile += (long long)gridDim.x * warps) {
     const bool ok = valid;
     const float t = target / W.out_scale;
 #pragma unroll
@@ -338,7 +338,7 @@ __global__ void __launch_bounds__(32 * kMaxGradWarps, 1)
     __syncwarp();
     // the next tile's samples arrive during the last product
     const long long next = tile + (long long)gridDim.x * warps;
-    if (next * kTile < hi) gather(next);
+    if (next * kTile < count) gather(next);
     // ---- weight gradient of layer 1: d1 (32 x samples) times x^T ----
 #pragma unroll 1
     for (int c = kTile / 2 * half; c < kTile / 2 * (half + 1); c += 4) {
@@ -390,9 +390,9 @@ __global__ void __launch_bounds__(32 * kMaxGradWarps, 1)
   }
 }
 
-// grad[e] = sum over blocks of partial[block][e] in FP64, added to grad[e] unless this is the
-// batch's first piece; with its last, grad[kTrainable] becomes the mean loss and, with kAdam, the
-// parameter takes its Adam update.  Eight entries (one 32-byte sector of a block's
+// grad[e] = sum over blocks of partial[block][e] in FP64, grad[kTrainable] the mean loss over
+// `count`; with kAdam also the Adam update of the parameter.  Of a batch in pieces (not kWhole),
+// every piece adds its sums to those of the pieces before it, and the last does the rest.  Eight entries (one 32-byte sector of a block's
 // row) per block and 16 groups of threads that take every 16th row each, then the 16 sums in
 // order.  One thread per entry summing all rows kept six blocks busy with a serial chain of
 // loads (16.3 us at 296 rows, Adam a launch of its own at 4.2 us).  128 threads of at most 32
@@ -405,11 +405,13 @@ struct AdamParams {
   float lr, beta1, beta2, eps;
   int step;
 };
+struct PieceOf {
+  bool first, last;
+};
 constexpr int kReduceEntries = 8, kReduceGroups = 16;
-template <bool kAdam>
+template <bool kAdam, bool kWhole>
 __global__ void __launch_bounds__(kReduceEntries * kReduceGroups, 16)
-    reduce_kernel(const float* partial, int blocks, long long count, bool first_piece, bool last_piece, double* grad,
-                  AdamParams ad) {
+    reduce_kernel(const float* partial, int blocks, long long count, PieceOf piece, double* grad, AdamParams ad) {
   __shared__ double part[kReduceGroups][kReduceEntries];
   const int entry = threadIdx.x % kReduceEntries, group = threadIdx.x / kReduceEntries;
   const int e = blockIdx.x * kReduceEntries + entry;
@@ -431,9 +433,9 @@ __global__ void __launch_bounds__(kReduceEntries * kReduceGroups, 16)
   s = 0.0;
 #pragma unroll
   for (int w = 0; w < kReduceGroups; ++w) s += part[w][entry];
-  if (!first_piece) s += grad[e];
-  grad[e] = last_piece && e == kTrainable ? s / (double)count : s;
-  if (!kAdam || !last_piece || e >= kTrainable) return;
+  if (!kWhole && !piece.first) s += grad[e];
+  grad[e] = (kWhole || piece.last) && e == kTrainable ? s / (double)count : s;
+  if (!kAdam || !(kWhole || piece.last) || e >= kTrainable) return;
   const float g = (float)s;
   const float mm = ad.beta1 * ad.m[e] + (1.f - ad.beta1) * g;
   const float vv = ad.beta2 * ad.v[e] + (1.f - ad.beta2) * g * g;
@@ -586,17 +588,19 @@ namespace {
 // more than kPieceSamples in pieces of that size.
 int run_gradient(psl_sgs_trainer* t, long long first, long long count, int random, uint32_t seed, const AdamParams* adam) {
   const unsigned int nb = (kTrainable + kReduceEntries) / kReduceEntries, threads = kReduceEntries * kReduceGroups;
-  for (long long lo = 0; lo < count; lo += kPieceSamples) {
-    const long long hi = std::min(count, lo + kPieceSamples);
-    const long long tiles = (hi - lo + kTile - 1) / kTile;
+  const bool whole = count <= kPieceSamples;
+  const auto reduce = adam ? (whole ? reduce_kernel<true, true> : reduce_kernel<true, false>)
+                           : (whole ? reduce_kernel<false, true> : reduce_kernel<false, false>);
+  for (long long at = 0; at < count; at += kPieceSamples) {
+    const long long samples = std::min(count - at, kPieceSamples), tiles = (samples + kTile - 1) / kTile;
     const int blocks = (int)std::min<long long>(kGradBlocks, tiles);
     const int warps = (int)std::min<long long>(kMaxGradWarps, (tiles + blocks - 1) / blocks);
     TRAIN_CUDA(launch_dependent(true, grad_kernel, dim3(blocks), 32 * warps, grad_smem(warps), t->stream,
-                                (const float*)t->params, (const float*)t->X, (const float*)t->T, t->count, first, lo, hi, count,
+                                (const float*)t->params, (const float*)t->X, (const float*)t->T, t->count, first + at, samples, count,
                                 random, seed, t->partial));
-    TRAIN_CUDA(launch_dependent(true, adam ? reduce_kernel<true> : reduce_kernel<false>, dim3(nb), threads, 0, t->stream,
-                                (const float*)t->partial, blocks, count, lo == 0, hi == count, t->grad,
-                                adam ? *adam : AdamParams{}));
+    const PieceOf piece{at == 0, at + samples == count};
+    TRAIN_CUDA(launch_dependent(true, reduce, dim3(nb), threads, 0, t->stream, (const float*)t->partial, blocks, count, piece,
+                                t->grad, adam ? *adam : AdamParams{}));
   }
   return PSL_OK;
 }
