@@ -33,11 +33,12 @@ using scalar_t = typename scalar_of<T>::type;
 
 // Two FP32 values in one packed operation (sm_100), each half rounded as the scalar operation.
 // The transforms pair lines of one cell that share their coefficients (x slots 0 and 2), so
-// the same arithmetic takes about 100 of 770 instructions per cell fewer and no more registers
-// (48 instead of 56 on twice-mapped rows).  FP32 grids in L2 are bound by issue and latency, and
-// large ones run at the power limit, where fewer instructions leave more clock: 128x64x64 sphere
-// with its drag 33.2 -> 30.1 us per step, 257x257x256 box 755 -> 714 us, refined 512x256x256
-// sphere 2.160 -> 2.110 ms, the 64-case batch 1.518 -> 1.457 ms.  FP64 keeps the scalar form.
+// the same arithmetic takes fewer instructions and no more registers (48 instead of 56 on
+// twice-mapped rows; with FlatIndex 730 instead of 776 executed per cell of the 512x256x256 grid).
+// FP32 grids in L2 are bound by issue and latency, and large ones run at the power limit, where
+// fewer instructions leave more clock: 128x64x64 sphere with its drag 33.2 -> 30.1 us per step,
+// 257x257x256 box 755 -> 714 us, the 64-case batch 1.518 -> 1.457 ms; coarse update of the
+// refined 512x256x256 sphere, with FlatIndex, 1.211 -> 1.174 ms.  FP64 keeps the scalar form.
 struct FPair {
   float2 v;
   __device__ __forceinline__ FPair() {}

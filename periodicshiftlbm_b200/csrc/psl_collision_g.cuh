@@ -247,7 +247,8 @@ PSL_HDI void bwd_full_w(T& a, T& b, T& c, const BwdAxis<T>& k, float wpm, float 
 // Two triples at once in packed FP32 (sm_100: one instruction, each half rounded as the scalar
 // operation; host builds take the halves one by one): the triples at x = -1 and x = +1 share
 // their coefficients and weights.  The 16-bit updates are bound by instruction issue beside
-// 64-byte row accesses; the pairs leave out about 46 instructions per cell, registers unchanged:
+// 64-byte row accesses; with FlatIndex the pairs leave out 42 of 669 executed instructions per cell
+// of the 512x256x256 grid, registers unchanged:
 // 251x117x125 BF16 grid 130.0 -> 127.2 us per step, refined 256x128x128 FP16 sphere
 // 232.4 -> 227.5 us, 129x129x128 FP16 box with the closure 105 -> 98.4 us.
 #if defined(__CUDACC__)

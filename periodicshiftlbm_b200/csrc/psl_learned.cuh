@@ -75,7 +75,7 @@ __device__ __forceinline__ void store_rows(const LearnedParams<S>& p, uint32_t c
   else store_cell_as<A>(p.ri, cell, f);
 }
 
-// 7 blocks of 128 per SM (72 registers; ptxas keeps ~40 bytes in local memory, L1-resident):
+// 7 blocks of 128 per SM (72 registers; ptxas keeps 8 to 72 bytes in local memory, L1-resident):
 // 1.2% faster than 6 blocks at 80 registers without spills, measured on the sphere case.
 template <typename S, bool kFlat, bool kStoreNu>
 __global__ void __launch_bounds__(kStepThreads, 7) step_learned_warp_kernel(const __grid_constant__ LearnedParams<S> p) {
