@@ -1101,6 +1101,10 @@ __global__ void __launch_bounds__(kForceThreads) force_partial_kernel(GridView<S
 // three components to `out`, device memory or mapped host memory, so no copy follows.
 // `done` counts the finished blocks and wraps to zero by itself with the last one, so a replayed
 // capture finds it as a direct call does.
+// What bounds it: latency (a few blocks, each a chain of loads, FP64 sums and barriers), then one
+// block's final sum.  Calls queued into pinned memory, against two kernels and a 24-byte copy:
+// radius 8 on 64^3 cells 17.6 -> 7.4 us, radius 60 on 256^3 cells (all 512 blocks) 86 -> 79 us.
+// Counted by a compare-and-swap loop the 512 blocks got through one at a time: 205 us.
 template <typename S>
 __global__ void __launch_bounds__(kForceThreads)
     force_kernel(const __grid_constant__ GridView<S> g, const uint8_t* marker, int nx, int ny, int i0, int j0, int k0, int si,
